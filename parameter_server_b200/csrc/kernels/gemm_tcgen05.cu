@@ -528,9 +528,11 @@ struct GemmProblemSet {
     int count;
     // Chain: problem i + 1 reads the output of problem i as its A operand (the layers of an MLP, forward or dgrad).
     // done[i * kMaxChainMTiles + m] counts the epilogue warps that have stored their part of an n-tile of row block m
-    // of problem i; a unit of problem i + 1 waits until all of row block m is there. Zeroed before every launch.
+    // of problem i; a unit of problem i + 1 waits until all of row block m is there. Zero between launches: the last CTA
+    // out puts the counters back, so that no memset stands in front of every launch; `left` counts the CTAs that are out.
     int chain;
     unsigned* done;
+    unsigned* left;
 };
 constexpr int kMaxChainMTiles = 1024;
 
@@ -1115,6 +1117,23 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ GemmProblemSet ps, unsigned* er
     // a pair leaves together: until here the peer may still signal this CTA's barriers or read its shared memory
     if constexpr (PAIR) cluster_sync_all();
     else __syncthreads();
+    if (ps.chain) {
+        // Every wait of this CTA has ended and its publisher has bumped its last counter (also after an error, when the
+        // waits ran out), so the CTA that finds all others out may reset the counters for the next launch.
+        if (threadIdx.x == 0) {
+            __threadfence();
+            *tmem_slot = atomicAdd(ps.left, 1u) + 1u == gridDim.x ? 1u : 0u;   // (the TMEM address is in a register by now)
+        }
+        __syncthreads();
+        if (*((volatile uint32_t*)tmem_slot) != 0u) {
+            const int m_blocks = (ps.M[0] + BM - 1) / BM + (PAIR ? 1 : 0);   // a pair's second half may lie past the last row
+            for (int i = threadIdx.x; i < ps.count * m_blocks; i += kThreads) {
+                const int p = i / m_blocks, m = i % m_blocks;
+                if (m < kMaxChainMTiles) ps.done[p * kMaxChainMTiles + m] = 0u;
+            }
+            if (threadIdx.x == 0) *ps.left = 0u;
+        }
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if constexpr (PAIR)
@@ -1399,6 +1418,7 @@ int gemm_bf16(const GemmOperand& A, const GemmOperand& B, const GemmEpilogue& ep
     ps.count = 1;
     ps.chain = 0;
     ps.done = nullptr;
+    ps.left = nullptr;
     ps.trace = g_gemm_trace;
     ps.epi_skip = epi_skip_env();
     const bool pair = pair_enabled() && !ag.enabled && M > BM;
@@ -1413,7 +1433,7 @@ void gemm_set_pair(int on) { g_gemm_pair = on ? 1 : 0; }
 
 void gemm_set_trace(void* device_buffer_of_256_u64) { g_gemm_trace = (unsigned long long*)device_buffer_of_256_u64; }
 
-int gemm_chain_scratch_words() { return kMaxGroup * kMaxChainMTiles; }
+int gemm_chain_scratch_words() { return kMaxGroup * kMaxChainMTiles + 1; }
 
 int gemm_bf16_grouped(const GemmOperand* A, const GemmOperand* B, const GemmEpilogue* ep, const int* M, const int* N,
                       const int* K, int count, unsigned* err_flag, double wait_limit_s, void* stream, unsigned* chain_done) {
@@ -1429,6 +1449,7 @@ int gemm_bf16_grouped(const GemmOperand* A, const GemmOperand* B, const GemmEpil
     ps.count = count;
     ps.chain = chain_done != nullptr ? 1 : 0;
     ps.done = chain_done;
+    ps.left = chain_done != nullptr ? chain_done + kMaxGroup * kMaxChainMTiles : nullptr;
     ps.trace = g_gemm_trace;
     ps.epi_skip = epi_skip_env();
     if (ps.chain) {
@@ -1438,7 +1459,12 @@ int gemm_bf16_grouped(const GemmOperand* A, const GemmOperand* B, const GemmEpil
             if (i > 0 && (K[i] != N[i - 1] || A[i].ptr != (const void*)ep[i - 1].out_bf16)) return -2;
         }
         if ((M[0] + BM - 1) / BM > kMaxChainMTiles) return -2;
-        cudaError_t e = cudaMemsetAsync(chain_done, 0, (size_t)count * kMaxChainMTiles * sizeof(unsigned), (cudaStream_t)stream);
+        // Under capture the scratch may have been made by a fill that is itself only captured, in a graph that need not be
+        // the first to be replayed: there every launch zeroes it.
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing((cudaStream_t)stream, &cap);
+        if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone)
+            e = cudaMemsetAsync(chain_done, 0, (size_t)gemm_chain_scratch_words() * sizeof(unsigned), (cudaStream_t)stream);
         if (e != cudaSuccess) return (int)e;
     }
     bool pair = false;

@@ -52,7 +52,7 @@ int gemm_bf16(const GemmOperand& A, const GemmOperand& B, const GemmEpilogue& ep
 // N >= 256, else 128 x 128). Meant for work that becomes available together, e.g. the weight gradients of all
 // layers of an MLP at the end of the backward pass. Same return codes as gemm_bf16.
 //
-// With `chain_done` (device scratch of gemm_chain_scratch_words() unsigned, zeroed by the call) the problems form a
+// With `chain_done` (device scratch of gemm_chain_scratch_words() unsigned, zero before the first call and left zero by every call) the problems form a
 // CHAIN: problem i + 1 takes the bf16 output of problem i as its A operand (the layers of an MLP in the forward
 // pass, or the dgrad sequence of the backward pass). All layers then run in this one launch: the work units are
 // ordered row block by row block, the epilogue counts the stored tiles of every row block, and the TMA producer

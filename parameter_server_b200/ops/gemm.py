@@ -116,7 +116,8 @@ def chain(layers, *, b_mn: bool = False, wait_limit_s: float = 2.0) -> None:
         raise ValueError("a chain holds 1..8 layers")
     dev = layers[0]["a"].device
     stream = torch.cuda.current_stream().cuda_stream
-    key = (dev.index or 0, stream)
+    # scratch made under capture is only filled when a graph runs: eager launches never share it
+    key = (dev.index or 0, stream, torch.cuda.is_current_stream_capturing())
     if key not in _chain_scratch:
         _chain_scratch[key] = torch.zeros(C.gemm_chain_scratch_words(), dtype=torch.int32, device=dev)
     probs = []
