@@ -50,6 +50,7 @@ struct TableView {
     unsigned* free_rows;      // stack of recycled rows
     int* free_count;
     unsigned long long* n_items;  // live keys
+    unsigned* erase_gen;      // bumped by every launch that may erase entries: a push whose plan is older looks its rows up again
     unsigned* touched_bits;   // 1 bit per row: row is in the sync-push touched list
     unsigned* touched_list;
     unsigned* touched_count;

@@ -93,6 +93,11 @@ SparseEngine::SparseEngine(GpuTable* table, const SparseEngineConfig& cfg) : tab
     const size_t o_res = carve((size_t)W * C_ * 4), o_new = carve((size_t)W * C_ * 4), o_next = carve((size_t)W * C_ * 4);
     // push, several ranks: per-CTA lists of chain heads and the sorted chain of every head
     const size_t o_heads = carve(W > 1 ? (size_t)W * C_ * 4 : 0), o_chain = carve(W > 1 ? (size_t)W * C_ * (size_t)W * 4 : 0);
+    // one GPU: sums of the keys that fill several work items of a push (zero between calls)
+    const size_t hot = W == 1 ? local_hot_rows((unsigned)N) : 0;
+    const size_t o_hsum = carve(hot * dim * 4), o_hcnt = carve(hot * 4), o_gen = carve(W == 1 ? 4 : 0);
+    const size_t o_idc = carve(W == 1 ? (size_t)N * 4 : 0);
+    const size_t o_big = carve(W == 1 ? (size_t)local_big_items((unsigned)N) * sizeof(uint4) : 0);
     const size_t o_rslot = carve(cfg_.replicate ? (size_t)W * C_ * 4 : 0), o_rnew = carve(cfg_.replicate ? (size_t)W * C_ * 4 : 0);
     const size_t o_cnt = carve(2 * 16 * 4), o_in = carve(2 * kMaxWorld * 4);
     const size_t o_ctl1 = carve(sizeof(KernelCtl)), o_ctl2 = carve(sizeof(KernelCtl));
@@ -115,6 +120,11 @@ SparseEngine::SparseEngine(GpuTable* table, const SparseEngineConfig& cfg) : tab
     ent_next_ = (unsigned*)(scratch_ + o_next);
     head_ids_ = (unsigned*)(scratch_ + o_heads);
     chain_buf_ = (unsigned*)(scratch_ + o_chain);
+    hot_sum_ = (float*)(scratch_ + o_hsum);
+    hot_cnt_ = (unsigned*)(scratch_ + o_hcnt);
+    plan_gen_ = (unsigned*)(scratch_ + o_gen);
+    big_items_ = scratch_ + o_big;
+    id_count_ = (unsigned*)(scratch_ + o_idc);
     rep_slot_ = (unsigned*)(scratch_ + o_rslot);
     rep_new_ = (unsigned*)(scratch_ + o_rnew);
     counters_ = (unsigned*)(scratch_ + o_cnt);
@@ -132,6 +142,8 @@ SparseEngine::SparseEngine(GpuTable* table, const SparseEngineConfig& cfg) : tab
     if (rc == 0) rc = fused_max_blocks(table_->device(), true, &max_pull_wide_, &max_push_wide_);
     if (rc != 0) throw std::runtime_error("SparseEngine: occupancy query failed");
     cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, table_->device());
+    if (W == 1 && local_prepare(&local_pull_small_, &local_pull_wide_, num_sms_) != 0)
+        throw std::runtime_error("SparseEngine: occupancy query failed");
     set_sm_budget(0, 0);
     cudaDeviceSynchronize();
     std::vector<void*> self(1, symm_->local());
@@ -255,6 +267,80 @@ void SparseEngine::fill_common(FusedArgs& a) const {
     a.rep_new = rep_new_;
 }
 
+void SparseEngine::fill_local(LocalArgs& a) const {
+    a.dim = table_->dim();
+    a.grads = nullptr;
+    a.table = table_->view_dev();
+    a.ctl = nullptr;
+    a.plan_ctl = ctl_pull_;
+    a.counters = counters_;
+    a.limit_ns = (unsigned long long)(cfg_.wait_limit_s * 1e9);
+    a.prof = profile_ ? prof_ : nullptr;
+    a.usage_mirror = table_->usage_mirror();
+    a.plan_gen = plan_gen_;
+    // the arrays of the general plan, which is never alive at the same time
+    a.id_of = pos_slot_;
+    a.rank_of = (unsigned*)inverse_;
+    a.push_row = (unsigned*)inverse_;
+    a.row_of = res_slot_;
+    a.slot_of_id = uniq_slot_;
+    a.count = id_count_;
+    a.info = (uint2*)agg_;
+    a.new_list = new_list_;
+    a.occ = ent_next_;
+    a.items = (uint4*)send_keys_;
+    a.big_items = (uint4*)big_items_;
+    a.key_copy = (long long*)agg_;
+    a.hot_sum = hot_sum_;
+    a.hot_cnt = hot_cnt_;
+}
+
+int SparseEngine::launch_general_pull(const long long* keys, uint32_t n, uint32_t bag_size, void* out, unsigned flags, void* stream) {
+    FusedArgs a;
+    fill_common(a);
+    a.flags = flags;
+    ++pull_epoch_;
+    a.ctl = ctl_pull_;
+    a.plan_ctl = ctl_pull_;
+    a.keys = keys;
+    a.n = n;
+    a.bag_size = bag_size;
+    a.out = out;
+    a.grads = nullptr;
+    a.hot_rows = 0;
+    int rc = launch_fused_pull(a, pull_blocks_, pull_wide_, stream);
+    ++launches_;
+    if (flags & FUSED_INSERT) table_->refresh_usage_async(stream);
+    return rc;
+}
+
+// The plan of the last pull as the general push reads it.
+Status SparseEngine::make_general_plan(void* stream) {
+    if (plan_kind_ == Plan::kGeneral) return Status::Ok();
+    int rc;
+    if (plan_kind_ == Plan::kLookup) {
+        // nothing was deduplicated: plan the keys that the lookup kept, still without inserting any
+        rc = launch_general_pull((const long long*)agg_, plan_n_, plan_bag_, nullptr, (plan_flags_ & FUSED_MEAN) | FUSED_PREPARE_PUSH, stream);
+    } else {
+        LocalArgs a;
+        fill_local(a);
+        a.n = plan_n_;
+        a.bag_size = plan_bag_;
+        a.flags = plan_flags_;
+        GeneralPlan g;
+        g.inverse = inverse_;
+        g.send_keys = send_keys_;
+        g.send_ret = send_ret_;
+        g.res_slot = res_slot_;
+        g.in_cnt = in_cnt_;
+        rc = launch_plan_to_general(a, g, num_sms_, stream);
+    }
+    if (rc != 0) return Status::Error(std::string("push plan launch: ") + cudaGetErrorString((cudaError_t)rc));
+    plan_kind_ = Plan::kGeneral;
+    plan_used_ = true;   // the aggregation rows are not zero
+    return Status::Ok();
+}
+
 Status SparseEngine::pull(const long long* keys, uint32_t n, uint32_t bag_size, void* out, unsigned flags,
                           void* stream) {
     if (failed_) return Status::Error("pull: the engine saw a fatal device status; call reset() on every rank first");
@@ -271,22 +357,31 @@ Status SparseEngine::pull(const long long* keys, uint32_t n, uint32_t bag_size, 
         if (!grown.ok() && grown.code() != StatusCode::OUT_OF_MEMORY) return grown;
         reserve = table_->reserve_rows(worst);
     }
-    FusedArgs a;
-    fill_common(a);
-    a.flags = flags;
-    ++pull_epoch_;
-    a.ctl = ctl_pull_;
-    a.plan_ctl = ctl_pull_;
-    a.keys = keys;
-    a.n = n;
-    a.bag_size = bag_size;
-    a.out = out;
-    a.grads = nullptr;
-    a.hot_rows = 0;
-    int rc = launch_fused_pull(a, pull_blocks_, pull_wide_, stream);
-    ++launches_;
-    if (flags & FUSED_INSERT) table_->refresh_usage_async(stream);
+    // One GPU: the local kernels; not for plans that the ordered sums or the replica log are made from, and not for a
+    // plan without insertion, whose missing keys only the general one can hold.
+    Plan kind = Plan::kGeneral;
+    if (cfg_.world == 1 && !deterministic_ && mirror_ == nullptr) {
+        if (flags & FUSED_INSERT) kind = Plan::kLocal;
+        else if (flags & FUSED_COPY_ROWS) kind = Plan::kLookup;
+    }
+    int rc;
+    if (kind == Plan::kGeneral) {
+        rc = launch_general_pull(keys, n, bag_size, out, flags, stream);
+    } else {
+        LocalArgs a;
+        fill_local(a);
+        a.keys = keys;
+        a.n = n;
+        a.bag_size = bag_size;
+        a.out = out;
+        a.flags = flags;
+        a.ctl = ctl_pull_;
+        if (kind == Plan::kLocal) rc = launch_local_pull(a, pull_wide_ ? std::min(local_pull_wide_, pull_blocks_) : local_pull_small_, pull_wide_, stream);
+        else rc = launch_local_lookup(a, pull_wide_ ? pull_blocks_ : num_sms_ * 8, pull_wide_, stream);
+        ++launches_;
+    }
     if (rc != 0) return Status::Error(std::string("fused_pull launch: ") + cudaGetErrorString((cudaError_t)rc));
+    plan_kind_ = kind;
     plan_keys_ = keys;
     plan_n_ = n;
     plan_bag_ = bag_size;
@@ -304,6 +399,24 @@ Status SparseEngine::push(const float* grads, uint32_t n_rows, const OptConfig& 
         return Status::InvalidConfig("push: gradient rows (" + std::to_string(n_rows) + ") != pulled bags (" +
                                      std::to_string(plan_n_ / plan_bag_) + ")");
     cudaSetDevice(table_->device());
+    if (plan_kind_ == Plan::kLocal && !deterministic_ && mirror_ == nullptr && !(flags & FUSED_AGG_READY)) {
+        LocalArgs a;
+        fill_local(a);
+        a.n = plan_n_;
+        a.bag_size = plan_bag_;
+        a.flags = plan_flags_ & FUSED_MEAN;
+        a.grads = grads;
+        a.opt = opt;
+        a.ctl = ctl_push_;
+        ++push_epoch_;
+        const int rc = launch_local_push(a, push_blocks_, push_wide_, (flags & FUSED_SYNC_PUSH) != 0, table_->n_opt_slots(), stream);
+        ++launches_;
+        if (rc != 0) return Status::Error(std::string("fused_push launch: ") + cudaGetErrorString((cudaError_t)rc));
+        plan_used_ = true;
+        return Status::Ok();
+    }
+    Status planned = make_general_plan(stream);
+    if (!planned.ok()) return planned;
     if (plan_used_ || !(plan_flags_ & FUSED_PREPARE_PUSH)) {
         // a plan pushed twice, or made by a pull that did not prepare a push: the aggregation rows must start
         // from zero
@@ -413,6 +526,7 @@ std::vector<uint64_t> SparseEngine::cta_stamps(int which, void* stream) {
 
 uint32_t SparseEngine::last_unique(void* stream) {
     cudaSetDevice(table_->device());
+    if (plan_valid_ && plan_kind_ == Plan::kLookup) make_general_plan(stream);   // a lookup counts nothing
     cudaStreamSynchronize((cudaStream_t)stream);
     KernelCtl h;
     cudaMemcpy(&h, ctl_pull_, sizeof(h), cudaMemcpyDeviceToHost);

@@ -10,6 +10,7 @@
 
 #include "../comm/symmetric.h"
 #include "../kernels/sparse_fused.h"
+#include "../kernels/sparse_local.h"
 #include "../storage/gpu_table.h"
 
 namespace psb {
@@ -90,6 +91,9 @@ public:
 
 private:
     void fill_common(FusedArgs& a) const;
+    void fill_local(LocalArgs& a) const;
+    int launch_general_pull(const long long* keys, uint32_t n, uint32_t bag_size, void* out, unsigned flags, void* stream);
+    Status make_general_plan(void* stream);
 
     GpuTable* table_;
     SparseEngineConfig cfg_;
@@ -129,6 +133,15 @@ private:
     void* sort_temp_ = nullptr;
     size_t sort_temp_bytes_ = 0;
     // last pull (the plan)
+    // Which plan the last pull left. One GPU: a pull that inserts leaves a local plan, one that does not a lookup (its
+    // keys only); with reproducible pushes or a mirror, and with several ranks, the general one. A push that finds
+    // another plan than the one it needs has it made first (make_general_plan).
+    enum class Plan { kGeneral, kLocal, kLookup };
+    Plan plan_kind_ = Plan::kGeneral;
+    unsigned *id_count_ = nullptr, *hot_cnt_ = nullptr, *plan_gen_ = nullptr;
+    float* hot_sum_ = nullptr;
+    void* big_items_ = nullptr;
+    int local_pull_small_ = 0, local_pull_wide_ = 0;
     const long long* plan_keys_ = nullptr;
     uint32_t plan_n_ = 0, plan_bag_ = 1;
     unsigned plan_flags_ = 0;

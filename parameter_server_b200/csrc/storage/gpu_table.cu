@@ -197,7 +197,13 @@ __device__ __forceinline__ void erase_slot(const TableView& t, uint64_t s, long 
     atomicAdd(n_erased, 1ull);
 }
 
+// Tells plans made before this launch that rows may have gone (read by the push, which is ordered behind it).
+__device__ __forceinline__ void bump_erase_gen(const TableView& t) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(t.erase_gen, 1u);
+}
+
 __global__ void erase_keys_kernel(TableView t, const long long* keys, uint64_t n, unsigned long long* n_erased) {
+    bump_erase_gen(t);
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         bool ins;
         const unsigned slot = table_find_or_insert(t, keys[i], false, &ins);
@@ -206,6 +212,7 @@ __global__ void erase_keys_kernel(TableView t, const long long* keys, uint64_t n
 }
 
 __global__ void erase_filter_kernel(TableView t, ShardFilter f, uint64_t cap, unsigned long long* n_erased) {
+    bump_erase_gen(t);
     for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < cap; s += (uint64_t)gridDim.x * blockDim.x) {
         const long long key = t.slots[s].key;
         if (key == kEmptyKey || key == kTombstoneKey) continue;
@@ -233,6 +240,7 @@ __device__ __forceinline__ float row_value(const TableView& t, const float* row,
 
 __global__ void scan_kernel(TableView t, ShardFilter f, DeviceScan sc, uint64_t cap, unsigned long long* n_erased,
                             double* stats /* count, sum, sum_sq, max_abs (bits) */) {
+    if (sc.pred_type >= 0) bump_erase_gen(t);
     const unsigned lane = threadIdx.x & 31u;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -342,6 +350,8 @@ __global__ void clear_aux_kernel(Slot* s, uint64_t n) {
         s[i].aux = kNoRow;
 }
 
+__global__ void bump_erase_gen_kernel(TableView t) { bump_erase_gen(t); }
+
 __global__ void rehash_kernel(const Slot* old_slots, uint64_t old_cap, Slot* new_slots, unsigned long long new_mask,
                               unsigned* status) {
     for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < old_cap; s += (uint64_t)gridDim.x * blockDim.x) {
@@ -398,7 +408,8 @@ GpuTable::GpuTable(const GpuTableConfig& cfg) : cfg_(cfg) {
     must(cudaMalloc(&scratch_, 64 * sizeof(unsigned long long)), "scratch");
     must(cudaMemset(scratch_, 0, 64 * sizeof(unsigned long long)), "scratch");
     // scratch layout (8-byte words): 0 n_items, 1 row_bump(u32), 2 free_count(i32), 3 touched_count(u32),
-    //                                4 op counter, 5 op status, 6 rows_avail(u32)
+    //                                4 op counter, 5 op status, 6 rows_avail(u32), 8..11 statistics,
+    //                                63 erase generation (u32; never reset, so that it differs after a clear too)
     n_items_ = scratch_ + 0;
     row_bump_ = (unsigned*)(scratch_ + 1);
     free_count_ = (int*)(scratch_ + 2);
@@ -568,6 +579,7 @@ TableView GpuTable::view() const {
     v.free_rows = free_rows_;
     v.free_count = free_count_;
     v.n_items = n_items_;
+    v.erase_gen = (unsigned*)(scratch_ + 63);
     v.touched_bits = touched_bits_;
     v.touched_list = touched_list_;
     v.touched_count = touched_count_;
@@ -754,7 +766,8 @@ Status GpuTable::clear(void* stream) {
     cudaSetDevice(cfg_.device);
     cudaStream_t s = (cudaStream_t)stream;
     fill_slots_kernel<<<grid_for(capacity_, 4), kThreads, 0, s>>>(slots_, capacity_);
-    PSB_CUDA_OK(cudaMemsetAsync(scratch_, 0, 64 * sizeof(unsigned long long), s));
+    PSB_CUDA_OK(cudaMemsetAsync(scratch_, 0, 63 * sizeof(unsigned long long), s));
+    bump_erase_gen_kernel<<<1, 32, 0, s>>>(view());
     PSB_CUDA_OK(cudaMemsetAsync(touched_bits_, 0, ((max_rows_ + 31) / 32) * 4, s));
     if (dirty_bits_) PSB_CUDA_OK(cudaMemsetAsync(dirty_bits_, 0, ((max_rows_ + 31) / 32) * 4, s));
     PSB_CUDA_OK(cudaMemcpyAsync(scratch_ + 6, &rows_avail_, sizeof(uint32_t), cudaMemcpyHostToDevice, s));

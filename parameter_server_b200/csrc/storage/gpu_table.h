@@ -69,6 +69,8 @@ public:
     Status reserve_exact(uint64_t n_new);
     // Enqueue a copy of the allocation counters into pinned host memory (read by reserve_rows).
     void refresh_usage_async(void* stream);
+    // The pinned words themselves (also a device address): a kernel that attaches rows may write them in place of the copy.
+    unsigned long long* usage_mirror() const { return (unsigned long long*)host_mirror_; }
     TableView view() const;
     // The same view in device memory, kept current by the table. Kernels whose launch is captured in a CUDA graph
     // read the table through this pointer, so that what the host changes between replays (a grown index, a larger
