@@ -8,9 +8,10 @@
 //      is kNoRow at rest. Whoever swaps first owns the key; everybody else reads the owner's number there. From here on
 //      all bookkeeping is in arrays indexed by that number. The occurrences are counted there, and the count returned
 //      tells each tile where its own begin.
-//   B  per number: the `aux` word goes back to rest, a new row is initialised, a key that occurs more than once gets a segment
+//   B  per number: a new row is initialised, a key that occurs more than once gets a segment
 //      of the occurrence list and work items for the push
-//   C  per position: row and segment of its key's number, then the rows are gathered and pooled
+//   C  per position: row and segment of its key's number; the `aux` words go back to rest; then the rows are gathered and
+//      pooled
 //   What bounds A is the number of scattered requests to the index (a few hundred MB: about 25 G/s for the whole GPU, whatever
 //   their width): one probe (1.5 with the chains), one swap and one reset per (tile, key), none per position.
 // local_push_kernel (plain launch, no barrier)
@@ -31,20 +32,20 @@ namespace psb {
 
 namespace {
 
-// How the occurrences of a repeated key are cut into work items of the push. Up to item_len go to one lane group; a key with
-// more has several items, and one with more than big_len is summed by whole CTAs, big_len occurrences each. Partial sums
-// of one key meet in one row of fp32 atomics, which costs about 80 ns each time: with one row per 32 occurrences the
-// hottest key of 4 Mi Zipf(1.05) keys (210 000 of them) took 548 us. Long items are a string of memory latencies
-// instead: with 1024 occurrences per CTA the 20 000 of a 213 Ki batch of dim 128 took 120 us, and a small batch ends
-// with its longest item. So the pieces grow with the batch.
+// How the occurrences of a repeated key are cut into work items of the push. Up to item_len go to one lane group, and a key with
+// more has several such items. Their sums meet in one row of fp32 atomics, which costs about 80 ns each time: with one
+// row per 32 occurrences the hottest key of 4 Mi Zipf(1.05) keys (210 000 of them) took 548 us. So a key with more than
+// big_min is summed by whole CTAs, big_len occurrences each. Those items are a string of memory latencies and CTA
+// barriers, 10 us each whatever their length (with big_min 128 the five hundred of a 213 Ki batch took 50 of the
+// push's 78 us on 96 SMs), and 1024 occurrences of dim 128 are 48 us: few of them, and no longer than the batch allows.
 struct Cut {
-    unsigned item_len, big_len;
+    unsigned item_len, big_min, big_len;
 };
-constexpr unsigned kMinItem = 16, kMinBig = 128;
+constexpr unsigned kMinItem = 16, kMinBig = 256;
 inline Cut cut_of(unsigned n) {
-    if (n < (1u << 18)) return {kMinItem, kMinBig};
-    if (n < (1u << 21)) return {32, 256};
-    return {32, 1024};
+    if (n < (1u << 18)) return {kMinItem, 1024, kMinBig};
+    if (n < (1u << 21)) return {32, 2048, 512};
+    return {32, 2048, 1024};
 }
 constexpr unsigned kDupRow = kRemoteRow;   // LocalArgs::push_row: the position's key is handled by a work item
 
@@ -56,7 +57,7 @@ struct Slot4 {
 // independent: each user re-checks what it needs with an atomic or after a barrier.
 __device__ __forceinline__ Slot4 ld_slot(const Slot* p) {
     unsigned a, b, c, d;
-    asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "l"(p) : "memory");
     Slot4 s;
     s.key = (long long)(((unsigned long long)b << 32) | a);
     s.row = c;
@@ -424,8 +425,6 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
                 c[q] = 0;
                 if (u >= a.n) continue;
                 c[q] = __ldcg(a.count + u);
-                const unsigned slot = __ldcg(a.slot_of_id + u);
-                if (slot != kNoSlot) T.slots[slot].aux = kNoRow;
             }
 #pragma unroll
             for (int q = 0; q < kU; ++q) {
@@ -438,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
             for (int q = 0; q < kU; ++q)
                 if (c[q] >= 2u) {
                     seg += c[q];
-                    if (c[q] <= a.big_len) {
+                    if (c[q] <= a.big_min) {
                         items += (c[q] + a.item_len - 1) / a.item_len;
                         multi += c[q] > a.item_len ? 1u : 0u;
                     }
@@ -467,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
 #pragma unroll
             for (int q = 0; q < kU; ++q) {
                 const bool dup = c[q] >= 2u;
-                const bool big = c[q] > a.big_len;
+                const bool big = c[q] > a.big_min;
                 const unsigned nch = dup && !big ? (c[q] + a.item_len - 1) / a.item_len : 0u;
                 unsigned mid = 0;
                 if (dup) {
@@ -537,6 +536,11 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
                 a.push_row[i] = pr;   // the same word as rank_of[i], which was read above
             }
         }
+    }
+    // The `aux` words go back to rest: scattered stores that nothing waits for here (in front of a barrier something would).
+    for (unsigned u = tid; u < a.n; u += nthreads) {
+        const unsigned slot = __ldcg(a.slot_of_id + u);
+        if (slot != kNoSlot) T.slots[slot].aux = kNoRow;
     }
     __syncthreads();
     if (a.flags & FUSED_COPY_ROWS) gather_bags(T, a, a.row_of, b_lo, b_hi);
@@ -962,6 +966,7 @@ int launch_local_pull(const LocalArgs& args, int max_blocks, bool wide, void* st
     LocalArgs a = args;
     const Cut cut = cut_of(a.n);
     a.item_len = cut.item_len;
+    a.big_min = cut.big_min;
     a.big_len = cut.big_len;
     void* params[] = {(void*)&a};
     // A small batch gets fewer CTAs: a barrier of few costs less than the work they would share. 64 keys per CTA (and at

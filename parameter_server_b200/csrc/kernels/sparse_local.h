@@ -6,7 +6,8 @@ namespace psb {
 
 struct LocalArgs {
     unsigned n, bag_size, dim, flags;
-    unsigned item_len, big_len;  // occurrences per work item of a lane group / of a CTA (set by launch_local_pull)
+    unsigned item_len, big_min, big_len;   // occurrences per work item of a lane group; a key with more than big_min is cut into
+                                           // CTA items of big_len (set by launch_local_pull)
     const long long* keys;       // [n]
     void* out;                   // [n / bag_size][dim] fp32, or bf16 with FUSED_OUT_BF16
     const float* grads;          // [n / bag_size][dim]
@@ -32,7 +33,7 @@ struct LocalArgs {
     unsigned* new_list;          // [N] slots whose rows this call attached
     unsigned* occ;               // [N] positions of the repeated keys, one contiguous segment per key
     uint4* items;                // [N/2] {row, first occurrence, length | items of the key << 8, 1 + hot index or 0}
-    uint4* big_items;            // [N/64 + 1] the same for keys that whole CTAs sum (length | items << 11)
+    uint4* big_items;            // [N/128 + 1] the same for keys that whole CTAs sum (length | items << 11)
     long long* key_copy;         // [N] lookup: the keys, in case a push follows
     float* hot_sum;              // [N/16 + 1][dim] sums of keys with several items: zero between calls
     unsigned* hot_cnt;           // [N/16 + 1] items of the key that have arrived: zero between calls
