@@ -338,12 +338,16 @@ class DLRM:
             self.side.wait_stream(main)
             with torch.cuda.stream(self.side):
                 self.sparse.pull(self.d_keys, out=self.emb); n_launch += 1
+                # the gradient buffer is first written by the head: cleared behind the pull, not in front of the bottom MLP,
+                # which on its few SMs is the longer branch
+                self.dense.zero_grads()  # torch fill kernels (not counted as own launches)
                 if self.stamps is not None:
                     self._mark("pull_done")
             # the GEMMs beside the pull: single CTAs (a pair needs two free SMs of one TPC) on the other SMs
             C.gemm_set_cta_limit(self.n_sms - self.pull_sms)
             C.gemm_set_pair(0)
-        self.dense.zero_grads()  # torch fill kernels (not counted as own launches)
+        if not self.overlap_fwd:
+            self.dense.zero_grads()  # torch fill kernels (not counted as own launches)
         self.loss.zero_()
         chk(C.cast_pad(self.d_dense.data_ptr(), B, cfg.num_dense, self.x16.data_ptr(), self.k_in, s)); n_launch += 1
         self._mark("zero_cast")
@@ -412,18 +416,29 @@ class DLRM:
                 dgrad.append(dict(a=dz, w=P[f"bot.w{i}"], mask=self.bot_act[i - 1], out=self.bot_dz[i - 1]))
         n_launch += self._dgrad_chain(dgrad)
         self._mark("bottom_dgrad")
-        G.grouped_wgrad(wg, split_k=self.split_k)
-        n_launch += (1 if any(x.shape[1] >= 256 for _, x, _ in wg) else 0) + (1 if any(x.shape[1] < 256 for _, x, _ in wg) else 0)
-        self._mark("wgrad")
-        G.bias_grads(bg); n_launch += (len(bg) + 7) // 8
-        self._mark("bias_grad")
-        if self.overlap:
-            C.gemm_set_cta_limit(0)
-            C.gemm_set_pair(1)
+        # With one rank the push is through soon after the bottom dgrad. Only the small gradient launches stay beside it; the
+        # branches join then, and the wide weight gradients get all SMs (54 us at batch 8192; 115 us on the 52 that the push
+        # leaves). With more ranks the push waits for its peers, and everything runs beside it.
+        joined = self.overlap and self.sparse.world == 1
+        wide = [it for it in wg if it[1].shape[1] >= 256]
+        if joined:
+            narrow = [it for it in wg if it[1].shape[1] < 256]
+            G.grouped_wgrad(narrow, split_k=self.split_k); n_launch += (len(narrow) + 7) // 8
+            G.bias_grads(bg); n_launch += (len(bg) + 7) // 8
+            self._mark("bias_grad")
+            self._end_push_overlap(main)
+            G.grouped_wgrad(wide, split_k=self.split_k); n_launch += (len(wide) + 7) // 8
+            self._mark("wgrad")
+        else:
+            G.grouped_wgrad(wg, split_k=self.split_k)
+            n_launch += (1 if wide else 0) + (1 if len(wide) < len(wg) else 0)
+            self._mark("wgrad")
+            G.bias_grads(bg); n_launch += (len(bg) + 7) // 8
+            self._mark("bias_grad")
+        if self.overlap and not joined:
             # join before the dense push: it waits for the other ranks like the sparse push does, and two kernels
             # that wait for peers must not compete for the same SMs
-            main.wait_stream(self.side)
-            self._mark("join_push")
+            self._end_push_overlap(main)
         if self.tail_overlap:
             # fork: the sparse push beside the dense push; both wait for their peers, on disjoint SMs
             self.side.wait_stream(main)
@@ -437,6 +452,13 @@ class DLRM:
         self._mark("dense_push")
         self.launches_per_step = n_launch
         return self.loss
+
+    def _end_push_overlap(self, main) -> None:
+        """The branch that runs beside the sparse push ends: the GEMMs get all SMs back once the push is through."""
+        C.gemm_set_cta_limit(0)
+        C.gemm_set_pair(1)
+        main.wait_stream(self.side)
+        self._mark("join_push")
 
     def _mlp_forward(self, x: torch.Tensor, acts, prefix: str) -> int:
         """``acts[i] = relu(acts[i-1] @ W_i^T + b_i)``; returns the number of launches."""
