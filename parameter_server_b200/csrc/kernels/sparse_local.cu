@@ -35,8 +35,8 @@ namespace {
 // more has several such items. Their sums meet in one row of fp32 atomics, which costs about 80 ns each time: with one
 // row per 32 occurrences the hottest key of 4 Mi Zipf(1.05) keys (210 000 of them) took 548 us. So a key with more than
 // big_min is summed by whole CTAs, big_len occurrences each. Those items are a string of memory latencies and CTA
-// barriers, 10 us each whatever their length (with big_min 128 the five hundred of a 213 Ki batch took 50 of the
-// push's 78 us on 96 SMs), and 1024 occurrences of dim 128 are 48 us: few of them, and no longer than the batch allows.
+// barriers (eight rows requested at a time), up to 10 us each even when short (with big_min 128 the five hundred of a 213 Ki batch took 50 of the
+// push's 78 us on 96 SMs): few of them, and no longer than the batch allows.
 struct Cut {
     unsigned item_len, big_min, big_len;
 };
@@ -47,6 +47,8 @@ inline Cut cut_of(unsigned n) {
     return {32, 2048, 1024};
 }
 constexpr unsigned kDupRow = kRemoteRow;   // LocalArgs::push_row: the position's key is handled by a work item
+
+constexpr unsigned kBehindOwner = 0x80000000u;   // LocalArgs::rank_of: counted from the end of the owner's own occurrences
 
 struct Slot4 {
     long long key;
@@ -343,7 +345,11 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
         }
 #pragma unroll
         for (int q = 0; q < kPer; ++q)
-            if (probes[q] == kDone) before[q] = atomicAdd(&a.count[owner[q]], s_cnt[s_list[(unsigned)q * kThreads + threadIdx.x]]);
+            if (probes[q] == kDone) {
+                // the owner's own occurrences come first and need no atomic (three entries in four, in a batch of 1 Mi)
+                const unsigned n_here = s_cnt[s_list[(unsigned)q * kThreads + threadIdx.x]];
+                before[q] = won[q] ? n_here : atomicAdd(&a.count[owner[q]], n_here) | kBehindOwner;
+            }
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
             const unsigned e = (unsigned)q * kThreads + threadIdx.x;
@@ -358,7 +364,11 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
                 }
                 a.info[t0 + e] = make_uint2(row < kRowPending ? row : kNoRow, 0u);
             }
-            if (e < tile_keys) a.slot_of_id[t0 + e] = won[q] ? eslot[q] : kNoSlot;
+            if (e < tile_keys) {
+                a.slot_of_id[t0 + e] = won[q] ? eslot[q] : kNoSlot;
+                a.own[t0 + e] = won[q] ? before[q] : 0u;
+            }
+            if (won[q]) before[q] = 0;
             // counters: one shared-memory atomic per warp, one global one per tile (new rows, rare, one per warp)
             const unsigned wm = __ballot_sync(0xffffffffu, won[q]), im = __ballot_sync(0xffffffffu, inserted[q]);
             const unsigned am = __ballot_sync(0xffffffffu, attached);
@@ -427,12 +437,13 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
                 c[q] = 0;
                 if (u >= a.n) continue;
                 c[q] = __ldcg(a.count + u);
+                const unsigned own = __ldcg(a.own + u);
+                if (c[q] != 0u) a.count[u] = 0;
+                c[q] += own;
             }
 #pragma unroll
             for (int q = 0; q < kU; ++q) {
                 const unsigned u = u0 + (unsigned)q * kThreads + threadIdx.x;
-                if (c[q] == 0u) continue;
-                a.count[u] = 0;
                 if (c[q] >= 2u) row[q] = __ldcg(&a.info[u].x);
             }
 #pragma unroll
@@ -530,7 +541,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
                 if (id[q] != kNoSlot) {
                     pr = row = f[q].x;
                     if (f[q].y != 0u) {
-                        a.occ[f[q].y - 1u + rank[q]] = i;
+                        const unsigned first = (rank[q] & kBehindOwner) ? __ldcg(a.own + id[q]) : 0u;
+                        a.occ[f[q].y - 1u + first + (rank[q] & ~kBehindOwner)] = i;
                         pr = kDupRow;
                     }
                 }
@@ -651,11 +663,17 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_push_kernel(c
                 float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (d < dim) {
                     auto add = [&](const float4& v) { acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w; };
+                    constexpr int kBig = 8;
                     unsigned j = lgroup;
-                    for (; j + 3 * lgroups < len; j += 4 * lgroups) {
-                        const unsigned p0 = occ[j], p1 = occ[j + lgroups], p2 = occ[j + 2 * lgroups], p3 = occ[j + 3 * lgroups];
-                        const float4 v0 = grad4(p0, d), v1 = grad4(p1, d), v2 = grad4(p2, d), v3 = grad4(p3, d);
-                        add(v0); add(v1); add(v2); add(v3);
+                    for (; j + (kBig - 1) * lgroups < len; j += kBig * lgroups) {
+                        unsigned q[kBig];
+                        float4 v[kBig];
+#pragma unroll
+                        for (int k = 0; k < kBig; ++k) q[k] = occ[j + k * lgroups];
+#pragma unroll
+                        for (int k = 0; k < kBig; ++k) v[k] = grad4(q[k], d);
+#pragma unroll
+                        for (int k = 0; k < kBig; ++k) add(v[k]);
                     }
                     for (; j < len; j += lgroups) add(grad4(occ[j], d));
                 }

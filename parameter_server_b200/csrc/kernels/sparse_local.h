@@ -23,12 +23,13 @@ struct LocalArgs {
     // ---- the plan, filled by a pull -------------------------------------------------------------------------------
     // A distinct key is known by the number of the entry that met it first: a place in the batch, below n.
     unsigned* id_of;             // [N] the key's number, of every position (kNoSlot: the index was full)
-    unsigned* rank_of;           // [N] how many earlier occurrences the position's key has ...
+    unsigned* rank_of;           // [N] how many earlier occurrences the position's key has (upper bit: behind the owner's) ...
     unsigned* push_row;          // [N] ... and, in the same memory, from phase C on: the table row of a key that occurs
                                  //     once, kRemoteRow where a work item covers the position, kNoRow without a row
     unsigned* row_of;            // [N] table row of every position (kNoRow: reads as the initial value)
     unsigned* slot_of_id;        // [N] table slot of the key with this number (kNoSlot: nobody's number)
-    unsigned* count;             // [N] occurrences of the key with this number: zero between calls
+    unsigned* own;               // [N] occurrences of the key with this number in the tile of that entry
+    unsigned* count;             // [N] its occurrences in all other tiles: zero between calls
     uint2* info;                 // [N] of the key with this number: table row (kNoRow: none), 1 + first of its occurrences or 0
     unsigned* new_list;          // [N] slots whose rows this call attached
     unsigned* occ;               // [N] positions of the repeated keys, one contiguous segment per key

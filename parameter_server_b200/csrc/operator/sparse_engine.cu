@@ -284,6 +284,7 @@ void SparseEngine::fill_local(LocalArgs& a) const {
     a.push_row = (unsigned*)inverse_;
     a.row_of = res_slot_;
     a.slot_of_id = uniq_slot_;
+    a.own = uniq_row_;
     a.count = id_count_;
     a.info = (uint2*)agg_;
     a.new_list = new_list_;
