@@ -382,8 +382,8 @@ def main():
             "parallelism": f"dp{world} + sparse rows sharded by key hash + dense slices (PS)",
             "vocab": "26 fields log-spaced 1e3..4e7 (~300M rows), rows created on first pull",
             "launch": "whole step replayed from one CUDA graph" if own["graph"] else "eager",
-            "streams": ("sparse pull beside the bottom MLP forward and sparse push beside bottom dgrad + weight / bias "
-                        "gradients (side stream; the GPU is split by SMs: pull %d / push %d SMs, GEMMs on the rest)" % (args.pull_sms, args.push_sms)) if own["overlap"] else (
+            "streams": ("sparse pull beside the bottom MLP forward and sparse push beside bottom dgrad + bias "
+                        "gradients, with two GPUs the weight gradients too (side stream; the GPU is split by SMs: pull %d / push %d SMs, GEMMs on the rest)" % (args.pull_sms, args.push_sms)) if own["overlap"] else (
                             ("pull beside the bottom MLP (%d SMs / rest); " % args.pull_sms if own.get("overlap_fwd") else "one stream; ") +
                             ("the sparse push (all SMs but 16) and the dense push (16 SMs) run side by side" if own.get("tail_overlap") else "")),
             "l2": "inputs larger than L2: ~55 MB of bf16 embedding rows gathered + ~109 MB of fp32 row gradients per step "

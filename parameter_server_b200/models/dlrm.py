@@ -179,8 +179,8 @@ class DLRM:
         # the layers of each MLP pass (bottom forward, top forward, top dgrad, bottom dgrad) run as one chained launch
         self.chain_gemms = bool(chain_gemms)
         # Overlap: the sparse pull runs on a side stream beside the bottom MLP forward, the sparse push beside the
-        # bottom dgrad + weight / bias gradients. The GPU is shared by SMs: a CTA of the fused sparse kernels and a
-        # CTA of the GEMM each fill an SM, so the pull (push) is launched on ``pull_sms`` (``push_sms``) SMs and the
+        # bottom dgrad + bias gradients (with two ranks the weight gradients too). The GPU is shared by SMs: a CTA of the
+        # fused sparse kernels and a CTA of the GEMM each fill an SM, so the pull (push) is launched on ``pull_sms`` (``push_sms``) SMs and the
         # GEMMs of the concurrent branch on the others, whichever kernel happens to start first.
         # Measured on B200: the split pays on one GPU (about 5 % of the step) and on two (2 %); from four ranks on the
         # pull and push spend much of their time waiting for peers, and SMs held by a waiting kernel are lost to the
