@@ -18,6 +18,18 @@ __global__ void iota_kernel(unsigned* p, unsigned n) {
 
 constexpr unsigned kBlock = 64;   // occurrences per block of the blocked sum
 
+// What the pull left behind. The counters live in the half selected by the parity of the pull's call epoch (device
+// memory: a launch replayed from a CUDA graph sees the current one). A pull that left early (a reserved key, a wait that
+// ran out) published no epoch: inverse map and counters are then of different calls, and the ids need not have runs. The
+// host learns of it at its next check only, so every pass looks at the status words itself, as the push does behind them.
+struct PlanWords {
+    const unsigned* counters;
+    const KernelCtl* pull;
+    const KernelCtl* push;
+    __device__ __forceinline__ bool cut_short() const { return (pull->status | push->status) != 0u; }
+    __device__ __forceinline__ unsigned n_uniq(unsigned n) const { return min(n, counters[(pull->epoch & 1u) * 16]); }
+};
+
 __device__ __forceinline__ float4 load_grad(const float* grads, unsigned pos, unsigned bag, unsigned dim, unsigned d, float scale) {
     float4 v = *(const float4*)(grads + (size_t)(pos / bag) * dim + d);
     if (scale != 1.0f) {
@@ -54,15 +66,13 @@ __device__ __forceinline__ float4 run_sum(const unsigned* __restrict__ sorted_po
 //
 // Pass 1, one thread per sorted entry: the first entry of a run writes the run's start (every id below n_uniq has a run,
 // so the next id's start is its end), and n behind the last.
-__global__ void __launch_bounds__(kThreads) run_starts_kernel(const unsigned* __restrict__ sorted_ids, unsigned n,
-                                                              const unsigned* __restrict__ counters, const unsigned* __restrict__ plan_epoch,
+__global__ void __launch_bounds__(kThreads) run_starts_kernel(const unsigned* __restrict__ sorted_ids, unsigned n, const PlanWords plan,
                                                               unsigned* __restrict__ starts) {
-    // the counters of a pull live in the half selected by the parity of the pull's call epoch (device memory: a
-    // launch replayed from a CUDA graph sees the current one)
-    const unsigned n_uniq = counters[(*plan_epoch & 1u) * 16];
+    if (plan.cut_short()) return;
+    const unsigned n_uniq = plan.n_uniq(n);
     for (unsigned j = blockIdx.x * kThreads + threadIdx.x; j < n; j += gridDim.x * kThreads) {
         const unsigned id = sorted_ids[j] & 0x7fffffffu;
-        if (j == 0 || (sorted_ids[j - 1] & 0x7fffffffu) != id) starts[id] = j;
+        if (id < n_uniq && (j == 0 || (sorted_ids[j - 1] & 0x7fffffffu) != id)) starts[id] = j;
         if (j == 0) starts[n_uniq] = n;
     }
 }
@@ -72,31 +82,32 @@ __global__ void __launch_bounds__(kThreads) run_starts_kernel(const unsigned* __
 // key's 20 000 occurrences of a 213 Ki batch of dim 128 to eight lane groups, and two binary searches per key (36 dependent
 // loads) came before: a step of 763 us, 285 us with these passes. What bounds them now is the latency of short kernels.
 __global__ void __launch_bounds__(kThreads) ordered_sum_kernel(const unsigned* __restrict__ starts,
-                                                              const unsigned* __restrict__ sorted_pos,
-                                                              const unsigned* __restrict__ counters,
-                                                              const unsigned* __restrict__ plan_epoch,
+                                                              const unsigned* __restrict__ sorted_pos, unsigned n, const PlanWords plan,
                                                               const float* __restrict__ grads, unsigned bag, unsigned dim,
                                                               float scale, float* __restrict__ agg, unsigned* __restrict__ long_cnt,
-                                                              uint4* __restrict__ long_runs, uint2* __restrict__ blocks) {
+                                                              uint4* __restrict__ long_runs, uint2* __restrict__ blocks, unsigned max_blocks) {
+    if (plan.cut_short()) return;
     const unsigned lanes = lanes_for_dim(dim);
     const unsigned tid = blockIdx.x * kThreads + threadIdx.x;
     const unsigned group = tid / lanes, ngroups = (gridDim.x * kThreads) / lanes, lane = tid % lanes;
-    const unsigned n_uniq = counters[(*plan_epoch & 1u) * 16];
+    const unsigned n_uniq = plan.n_uniq(n);
     unsigned nlo = 0, nend = 0;
     if (group < n_uniq) { nlo = starts[group]; nend = starts[group + 1]; }
     for (unsigned u = group; u < n_uniq; u += ngroups) {
         const unsigned lo = nlo, end = nend;
         if (u + ngroups < n_uniq) { nlo = starts[u + ngroups]; nend = starts[u + ngroups + 1]; }
+        if (lo >= end || end > n) continue;   // an id without a run: nothing below may leave the arrays for it
         if (end - lo > kBlock) {
             const unsigned nblk = (end - lo + kBlock - 1) / kBlock;
             unsigned base = 0;
             if (lane == 0) {
                 base = atomicAdd(long_cnt + 1, nblk);   // work items, and rows of the scratch area for their sums
-                long_runs[atomicAdd(long_cnt, 1u)] = make_uint4(u, base, nblk, 0u);
+                if (base + nblk <= max_blocks) long_runs[atomicAdd(long_cnt, 1u)] = make_uint4(u, base, nblk, 0u);
             }
             const unsigned wl = threadIdx.x & 31u, gl0 = wl / lanes * lanes;
             const unsigned gmask = (lanes >= 32u ? 0xffffffffu : ((1u << lanes) - 1u)) << gl0;
             base = __shfl_sync(gmask, base, gl0);
+            if (base + nblk > max_blocks) continue;
             for (unsigned k = lane; k < nblk; k += lanes) blocks[base + k] = make_uint2(lo + k * kBlock, min(end, lo + (k + 1) * kBlock));
             continue;
         }
@@ -106,14 +117,15 @@ __global__ void __launch_bounds__(kThreads) ordered_sum_kernel(const unsigned* _
 }
 
 // Pass 3, one lane group per block of a long run.
-__global__ void __launch_bounds__(kThreads) block_sum_kernel(const unsigned* __restrict__ sorted_pos, const float* __restrict__ grads,
+__global__ void __launch_bounds__(kThreads) block_sum_kernel(const unsigned* __restrict__ sorted_pos, unsigned n, const float* __restrict__ grads,
                                                             unsigned bag, unsigned dim, float scale, const unsigned* __restrict__ long_cnt,
-                                                            const uint2* __restrict__ blocks, float* __restrict__ partials) {
+                                                            const uint2* __restrict__ blocks, unsigned max_blocks, float* __restrict__ partials) {
     const unsigned lanes = lanes_for_dim(dim);
     const unsigned tid = blockIdx.x * kThreads + threadIdx.x;
-    const unsigned n_blocks = long_cnt[1], lane = tid % lanes;
+    const unsigned n_blocks = min(long_cnt[1], max_blocks), lane = tid % lanes;
     for (unsigned k = tid / lanes; k < n_blocks; k += (gridDim.x * kThreads) / lanes) {
         const uint2 b = blocks[k];
+        if (b.x >= b.y || b.y > n) continue;
         for (unsigned d = lane * 4; d < dim; d += lanes * 4)
             *(float4*)(partials + (size_t)k * dim + d) = run_sum(sorted_pos, b.x, b.y, grads, bag, dim, d, scale);
     }
@@ -152,6 +164,7 @@ namespace {
 // layout of the temporary storage after the identity permutation and cub's own scratch
 struct Scratch {
     size_t counters, starts, runs, blocks, partials, total;
+    unsigned max_blocks;
 };
 Scratch scratch_layout(unsigned max_n, unsigned dim, size_t cub_bytes) {
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
@@ -161,9 +174,9 @@ Scratch scratch_layout(unsigned max_n, unsigned dim, size_t cub_bytes) {
     const size_t max_long = (size_t)max_n / kBlock + 1;                 // runs longer than kBlock
     l.starts = o; o += up(((size_t)max_n + 1) * sizeof(unsigned));
     l.runs = o; o += up(max_long * sizeof(uint4));
-    const size_t max_blocks = 2 * max_long + 1;                         // sum of ceil(len / kBlock) over the long runs
-    l.blocks = o; o += up(max_blocks * sizeof(uint2));
-    l.partials = o; o += up(max_blocks * (size_t)dim * sizeof(float));
+    l.max_blocks = (unsigned)(2 * max_long + 1);                        // sum of ceil(len / kBlock) over the long runs
+    l.blocks = o; o += up(l.max_blocks * sizeof(uint2));
+    l.partials = o; o += up(l.max_blocks * (size_t)dim * sizeof(float));
     l.total = o;
     return l;
 }
@@ -177,9 +190,9 @@ size_t cub_sort_bytes(unsigned max_n) {
 
 size_t ordered_segment_sum_temp_bytes(unsigned max_n, unsigned dim) { return scratch_layout(max_n, dim, cub_sort_bytes(max_n)).total; }
 
-int ordered_segment_sum(const int* inverse, unsigned n, unsigned max_n, const unsigned* counters, const unsigned* plan_epoch,
-                        const float* grads, unsigned bag, unsigned dim, float scale, float* agg, unsigned* sorted_ids,
-                        unsigned* sorted_pos, void* temp, size_t temp_bytes, void* stream) {
+int ordered_segment_sum(const int* inverse, unsigned n, unsigned max_n, const unsigned* counters, const KernelCtl* pull_ctl,
+                        const KernelCtl* push_ctl, const float* grads, unsigned bag, unsigned dim, float scale, float* agg,
+                        unsigned* sorted_ids, unsigned* sorted_pos, void* temp, size_t temp_bytes, void* stream) {
     if (n == 0) return 0;
     if (n > max_n) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
@@ -193,6 +206,7 @@ int ordered_segment_sum(const int* inverse, unsigned n, unsigned max_n, const un
     uint4* long_runs = (uint4*)((char*)temp + l.runs);
     uint2* blocks = (uint2*)((char*)temp + l.blocks);
     float* partials = (float*)((char*)temp + l.partials);
+    const PlanWords plan = {counters, pull_ctl, push_ctl};
     cudaError_t e = cudaMemsetAsync(long_cnt, 0, 8, s);
     if (e != cudaSuccess) return (int)e;
     iota_kernel<<<148 * 2, kThreads, 0, s>>>(iota, n);
@@ -206,11 +220,12 @@ int ordered_segment_sum(const int* inverse, unsigned n, unsigned max_n, const un
     const unsigned long long want = ((unsigned long long)n * lanes + kThreads - 1) / kThreads;
     const unsigned grid = (unsigned)(want < 148 * 16 ? want : 148 * 16);
     const unsigned grid_n = (unsigned)(((unsigned long long)n + kThreads - 1) / kThreads);
-    run_starts_kernel<<<grid_n < 148 * 8 ? grid_n : 148 * 8, kThreads, 0, s>>>(sorted_ids, n, counters, plan_epoch, starts);
-    ordered_sum_kernel<<<grid, kThreads, 0, s>>>(starts, sorted_pos, counters, plan_epoch, grads, bag, dim, scale, agg, long_cnt, long_runs, blocks);
+    run_starts_kernel<<<grid_n < 148 * 8 ? grid_n : 148 * 8, kThreads, 0, s>>>(sorted_ids, n, plan, starts);
+    ordered_sum_kernel<<<grid, kThreads, 0, s>>>(starts, sorted_pos, n, plan, grads, bag, dim, scale, agg, long_cnt, long_runs, blocks, l.max_blocks);
     // at most n / kBlock + (long runs) blocks, and a long run has more than kBlock entries
     const unsigned long long want_blocks = (2ull * n / kBlock * lanes + kThreads - 1) / kThreads + 1;
-    block_sum_kernel<<<(unsigned)(want_blocks < 148 * 8 ? want_blocks : 148 * 8), kThreads, 0, s>>>(sorted_pos, grads, bag, dim, scale, long_cnt, blocks, partials);
+    block_sum_kernel<<<(unsigned)(want_blocks < 148 * 8 ? want_blocks : 148 * 8), kThreads, 0, s>>>(sorted_pos, n, grads, bag, dim, scale, long_cnt, blocks, l.max_blocks,
+                                                                                                             partials);
     const unsigned long long want_runs = ((unsigned long long)n / kBlock * lanes + kThreads - 1) / kThreads + 1;
     fold_blocks_kernel<<<(unsigned)(want_runs < 148 * 2 ? want_runs : 148 * 2), kThreads, 0, s>>>(dim, long_cnt, long_runs, partials, agg);
     return (int)cudaGetLastError();

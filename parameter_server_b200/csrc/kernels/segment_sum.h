@@ -15,16 +15,18 @@
 
 namespace psb {
 
+struct KernelCtl;
+
 // Bytes of temporary device storage needed for batches of up to max_n positions.
 size_t ordered_segment_sum_temp_bytes(unsigned max_n, unsigned dim);
 
-// inverse[n]: unique id of every position; counters / plan_epoch: the pull's counter block ([2][16] words, word 0 of
-// a half = number of unique ids) and the device word whose parity selects the half; grads:
-// [n / bag][dim]; agg: [n_uniq][dim] output. `scale` multiplies every gradient (mean pooling), 1 for none.
+// inverse[n]: unique id of every position; counters: the pull's counter block ([2][16] words, word 0 of a half = number
+// of unique ids; the parity of the pull's epoch selects the half); pull_ctl / push_ctl: the two control blocks, nothing
+// is summed when either holds a fatal status (the map and the counters then belong together no more); grads: [n / bag][dim]; agg: [n_uniq][dim] output. `scale` multiplies every gradient (mean pooling), 1 for none.
 // sorted_ids / sorted_pos: device scratch of max_n unsigned each; temp: ordered_segment_sum_temp_bytes(max_n, dim)
 // bytes (max_n = the size the storage was made for, n <= max_n). Returns 0 or a cudaError_t.
-int ordered_segment_sum(const int* inverse, unsigned n, unsigned max_n, const unsigned* counters, const unsigned* plan_epoch,
-                        const float* grads, unsigned bag, unsigned dim, float scale, float* agg, unsigned* sorted_ids,
-                        unsigned* sorted_pos, void* temp, size_t temp_bytes, void* stream);
+int ordered_segment_sum(const int* inverse, unsigned n, unsigned max_n, const unsigned* counters, const KernelCtl* pull_ctl,
+                        const KernelCtl* push_ctl, const float* grads, unsigned bag, unsigned dim, float scale, float* agg,
+                        unsigned* sorted_ids, unsigned* sorted_pos, void* temp, size_t temp_bytes, void* stream);
 
 }  // namespace psb

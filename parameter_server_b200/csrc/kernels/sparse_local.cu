@@ -923,7 +923,9 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_lookup_kernel
 }
 
 // ---- a plan of the local pull turned into one of the general push ---------------------------------------------------
+// After a pull that left early there is no plan: its arrays are of an earlier call, perhaps of the general kernel's.
 __global__ void __launch_bounds__(256) plan_entries_kernel(const LocalArgs a, const GeneralPlan g, unsigned* n_entries) {
+    if (a.plan_ctl->status != 0u) return;
     for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < a.n; i += gridDim.x * 256) {
         const unsigned slot = a.slot_of_id[i];
         if (slot == kNoSlot) continue;
@@ -935,6 +937,7 @@ __global__ void __launch_bounds__(256) plan_entries_kernel(const LocalArgs a, co
     }
 }
 __global__ void __launch_bounds__(256) plan_positions_kernel(const LocalArgs a, const GeneralPlan g, unsigned* n_entries) {
+    if (a.plan_ctl->status != 0u) return;
     for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < a.n; i += gridDim.x * 256) {
         const unsigned id = a.id_of[i];
         unsigned u, bit = 0;
@@ -950,6 +953,7 @@ __global__ void __launch_bounds__(256) plan_positions_kernel(const LocalArgs a, 
     }
 }
 __global__ void plan_finish_kernel(const LocalArgs a, const GeneralPlan g, unsigned* n_entries) {
+    if (a.plan_ctl->status != 0u) return;
     const unsigned par = a.plan_ctl->epoch & 1u, n = *n_entries;
     *n_entries = 0;
     a.counters[par * 16] = n;

@@ -426,7 +426,7 @@ Status SparseEngine::push(const float* grads, uint32_t n_rows, const OptConfig& 
     if (deterministic_ && !(flags & FUSED_AGG_READY)) {
         // position-ordered sums of the duplicates, then the fused kernel without its own (atomic) segment sum
         const float scale = (plan_flags_ & FUSED_MEAN) && plan_bag_ > 1 ? 1.0f / (float)plan_bag_ : 1.0f;
-        int rc0 = ordered_segment_sum(inverse_, plan_n_, cfg_.max_keys, counters_, &ctl_pull_->epoch, grads, plan_bag_, table_->dim(), scale,
+        int rc0 = ordered_segment_sum(inverse_, plan_n_, cfg_.max_keys, counters_, ctl_pull_, ctl_push_, grads, plan_bag_, table_->dim(), scale,
                                       agg_, sorted_ids_, sorted_pos_, sort_temp_, sort_temp_bytes_, stream);
         if (rc0 != 0) return Status::Error(std::string("ordered_segment_sum: ") + cudaGetErrorString((cudaError_t)rc0));
         flags |= FUSED_AGG_READY;
