@@ -62,3 +62,24 @@ def test_reproducible_push_behind_a_refused_pull(how, reserved):
         step(g, c, hot)
         step(g, c, keys[:100])
     same(g, c, hot)
+
+
+def test_pair_capacity_below_the_batch_on_one_gpu():
+    """Exact up to ``pair_capacity`` distinct keys whatever the batch's length, an error status beyond."""
+    g, c = tables(pair_capacity=1000)
+    keys = torch.arange(4096) % 1000 * 7 + 3
+    few = torch.arange(1000) * 7 + 10                 # short enough for a plan with an entry per position
+    for k in (keys, few, keys.flip(0)):
+        step(g, c, k)
+        assert torch.equal(g.pull(k.cuda(), insert=False, for_push=False).cpu(), c.pull(k))
+    step(g, c, keys, bag=4)
+    grads = whole(4096, 16)
+    g.pull(keys.cuda(), insert=False, for_push=False); c.pull(keys)
+    g.push(grads.cuda()); c.push(grads)
+    g.check()
+    same(g, c, torch.cat([keys, few]))
+    g.pull((torch.arange(1001) * 7 + 3).cuda())
+    st = g.status()
+    assert st.code() == StatusCode.ERROR and "pair_capacity" in st.msg()
+    g.reset()
+    step(g, c, keys)
