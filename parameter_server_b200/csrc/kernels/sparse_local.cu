@@ -202,6 +202,28 @@ __device__ __forceinline__ void gather_bags(const TableView& T, const LocalArgs&
     }
 }
 
+// A reserved key refuses the whole batch, but it is found when other CTAs have inserted their keys (a barrier in front of
+// the first insertion cost 1.5 us of a step of 8192 keys, 4.7 us of 65536). The refused call takes them out again: a slot
+// that was empty before the call ends no chain but those of the call's own keys, so it may be empty again. Rows go
+// to the free stack; whoever gets one initialises it.
+__device__ __noinline__ void undo_inserts(const TableView* table, const unsigned* new_rows, const unsigned* new_keys, const unsigned* counts,
+                                          const unsigned* slot_of_id, unsigned n) {
+    const TableView& T = *table;
+    const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+    const unsigned n_rows = __ldcg(counts), n_keys = __ldcg(counts + 1);
+    for (unsigned j = tid; j < n_rows; j += nthreads) {
+        const unsigned slot = __ldcg(new_rows + j), row = __ldcg(&T.slots[slot].row);
+        T.slots[slot].row = kNoRow;
+        T.free_rows[atomicAdd(T.free_count, 1)] = row;
+    }
+    for (unsigned j = tid; j < n_keys; j += nthreads) T.slots[__ldcg(new_keys + j)].key = kEmptyKey;
+    for (unsigned u = tid; u < n; u += nthreads) {
+        const unsigned slot = __ldcg(slot_of_id + u);
+        if (slot != kNoSlot) T.slots[slot].aux = kNoRow;
+    }
+    if (tid == 0) atomicAdd(T.n_items, 0ull - n_keys);
+}
+
 // Tile of the shared-memory dedup: positions per tile, and twice as many table slots (load at most one half).
 template <int kThreads> struct Tile {
     static constexpr int kPer = kThreads >= 1024 ? 2 : 4;
@@ -228,7 +250,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
     if (ld_acquire_gpu(&a.ctl->status) != 0u) return;
     const unsigned epoch = *((volatile unsigned*)&a.ctl->epoch) + 1u;
     const unsigned par = epoch & 1u;
-    unsigned* cnt = a.counters + par * 16;   // 0 distinct, 1 new rows, 2 occurrence list, 3 work items, 5 keys with several items
+    unsigned* cnt = a.counters + par * 16;   // see LocalArgs::counters
     const TableView T = *a.table;
     PROF(0);
     PROF_CTA(0);
@@ -369,18 +391,19 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
                 a.own[t0 + e] = won[q] ? before[q] : 0u;
             }
             if (won[q]) before[q] = 0;
-            // counters: one shared-memory atomic per warp, one global one per tile (new rows, rare, one per warp)
+            // counters: one shared-memory atomic per warp, one global one per tile (new rows and entries, rare, one per warp)
             const unsigned wm = __ballot_sync(0xffffffffu, won[q]), im = __ballot_sync(0xffffffffu, inserted[q]);
             const unsigned am = __ballot_sync(0xffffffffu, attached);
             if (wlane == 0) {
                 if (wm) atomicAdd(&s_sum[0], (unsigned)__popc(wm));
                 if (im) atomicAdd(&s_sum[1], (unsigned)__popc(im));
             }
-            if (am) {
-                unsigned ab = 0;
-                if (wlane == 0) ab = atomicAdd(&cnt[1], (unsigned)__popc(am));
+            if (am | im) {
+                unsigned long long ab = 0;
+                if (wlane == 0) ab = atomicAdd((unsigned long long*)&cnt[8], (unsigned long long)__popc(im) << 32 | (unsigned)__popc(am));
                 ab = __shfl_sync(0xffffffffu, ab, 0);
-                if (attached) a.new_list[ab + __popc(am & lt)] = eslot[q];
+                if (attached) a.new_list[(unsigned)ab + __popc(am & lt)] = eslot[q];
+                if (inserted[q]) a.occ[(unsigned)(ab >> 32) + __popc(im & lt)] = eslot[q];   // for undo_inserts
             }
         }
         __syncthreads();   // every entry has read its key
@@ -410,16 +433,21 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
         }
         __syncthreads();   // the tables are emptied for the next tile
     }
+    if (reserved) cnt[7] = 1u;
     PROF_CTA(1);
     unsigned gen = grid_arrive(a.ctl, nblocks);
     if (!grid_wait(a.ctl, gen, a.limit_ns, W_P1)) return;
-    // reported only now: a CTA that had not started yet would take the word for an earlier call's and leave
-    if (reserved) set_status(a.ctl, kStError, W_RESERVED_KEY);
+    if (*((volatile unsigned*)&cnt[7]) != 0u) {
+        undo_inserts(a.table, a.new_list, a.occ, cnt + 8, a.slot_of_id, a.n);
+        // reported only now: a CTA that had not started yet would take the word for an earlier call's and leave
+        if (tid == 0) set_status(a.ctl, kStError, W_RESERVED_KEY);
+        return;
+    }
     PROF(1);
     PROF(2);
 
     // ---- B ------------------------------------------------------------------------------------------------------
-    const unsigned n_new = *((volatile unsigned*)&cnt[1]);
+    const unsigned n_new = *((volatile unsigned*)&cnt[8]);
     if (blockIdx.x == 0 && threadIdx.x == 0 && a.usage_mirror != nullptr) {
         // the allocation counters that the host's next reservation reads (no copy engine, no extra launch)
         a.usage_mirror[0] = *((volatile unsigned*)T.row_bump);

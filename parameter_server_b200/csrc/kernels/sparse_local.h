@@ -14,8 +14,9 @@ struct LocalArgs {
     const TableView* table;      // device memory, see FusedArgs::table
     KernelCtl* ctl;
     const KernelCtl* plan_ctl;   // push: control block of the pull family
-    unsigned* counters;          // [2][16] per epoch parity of the pull: 0 distinct keys, 1 new rows, 2 occurrences listed,
-                                 // 3 work items, 5 keys with several items, 6 work items of whole CTAs
+    unsigned* counters;          // [2][16] per epoch parity of the pull: 0 distinct keys, 2 occurrences listed,
+                                 // 3 work items, 5 keys with several items, 6 work items of whole CTAs, 7 a reserved key was
+                                 // met, 8 new rows and 9 new entries of the index (one 64-bit word)
     unsigned long long limit_ns;
     unsigned long long* prof;
     unsigned long long* usage_mirror;   // pinned host words {row_bump, free_count}
@@ -32,7 +33,8 @@ struct LocalArgs {
     unsigned* count;             // [N] its occurrences in all other tiles: zero between calls
     uint2* info;                 // [N] of the key with this number: table row (kNoRow: none), 1 + first of its occurrences or 0
     unsigned* new_list;          // [N] slots whose rows this call attached
-    unsigned* occ;               // [N] positions of the repeated keys, one contiguous segment per key
+    unsigned* occ;               // [N] positions of the repeated keys, one contiguous segment per key (phase A: slots of
+                                 //     the keys that this call inserted)
     uint4* items;                // [N/2] {row, first occurrence, length | items of the key << 8, 1 + hot index or 0}
     uint4* big_items;            // [N/128 + 1] the same for keys that whole CTAs sum (length | items << 11)
     long long* key_copy;         // [N] lookup: the keys, in case a push follows

@@ -83,3 +83,67 @@ def test_pair_capacity_below_the_batch_on_one_gpu():
     assert st.code() == StatusCode.ERROR and "pair_capacity" in st.msg()
     g.reset()
     step(g, c, keys)
+
+
+@pytest.mark.parametrize("n,at,sms,bag", [(1, 0, 0, 1), (300, 299, 0, 1), (9000, 8999, 1, 1), (9000, 4500, 3, 3), (70000, 69999, 0, 1), (70000, 0, 5, 7), (70000, 35000, 1, 70000)])
+@pytest.mark.parametrize("call", ["pull", "plan"])
+def test_a_refused_batch_leaves_the_table_alone(n, at, sms, bag, call):
+    """A reserved key anywhere (one tile or several per CTA): none of the batch's other keys is inserted."""
+    g, c = tables(max_keys=70000)
+    if sms:
+        g.set_sm_budget(sms, sms)
+    old = torch.arange(500) * 13 + 1
+    step(g, c, old)
+    fresh = torch.arange(n) * 13 + 2
+    bad = fresh.clone()
+    bad[at] = RESERVED[n % 2]
+    getattr(g, call)(bad.cuda(), bag)
+    g.push(torch.ones(n // bag, 16, device="cuda"))
+    st = g.status()
+    assert st.code() == StatusCode.ERROR and "reserved" in st.msg()
+    assert g.size() == 500 and not g.get_rows(fresh.cuda())[1].any()
+    same(g, c, old)
+    g.reset()
+    step(g, c, fresh, bag)
+    step(g, c, old)
+    same(g, c, torch.cat([old, fresh]))
+
+
+@pytest.mark.parametrize("n,at,sms,bag", [(1, 0, 0, 1), (300, 299, 0, 1), (9000, 8999, 1, 1), (9000, 4500, 3, 3), (70000, 69999, 0, 1), (70000, 0, 5, 7), (70000, 35000, 1, 70000)])
+@pytest.mark.parametrize("call", ["pull", "plan"])
+def test_a_refused_batch_leaves_the_table_alone(n, at, sms, bag, call):
+    """A reserved key anywhere (one tile or several per CTA): none of the batch's other keys stays in the table."""
+    g, c = tables(max_keys=70000)
+    if sms:
+        g.set_sm_budget(sms, sms)
+    old = torch.arange(500) * 13 + 1
+    step(g, c, old)
+    fresh = torch.arange(n) * 13 + 2
+    bad = torch.cat([fresh, fresh[:n // 3]])[-n:]       # some keys twice
+    bad[at] = RESERVED[n % 2]
+    getattr(g, call)(bad.cuda(), bag)
+    g.push(torch.ones(n // bag, 16, device="cuda"))
+    st = g.status()
+    assert st.code() == StatusCode.ERROR and "reserved" in st.msg()
+    assert g.size() == 500 and not g.get_rows(fresh.cuda())[1].any()
+    same(g, c, old)
+    g.reset()
+    step(g, c, fresh, bag)
+    step(g, c, old)
+    same(g, c, torch.cat([old, fresh]))
+
+
+def test_a_refused_batch_gives_back_the_rows_of_an_exhausted_pool():
+    g, c = tables(max_keys=4096, slab_shift=11)
+    old = torch.arange(500) * 13 + 1
+    g.reserve(500, exact=True)
+    g.set_rows(old.cuda(), torch.ones(500, 32).cuda()); c.set_rows(old, torch.ones(500, 32))
+    g.table.set_limits(1, 1)                            # no further slab: 2048 rows
+    bad = torch.arange(4000) * 13 + 2
+    bad[17] = RESERVED[0]
+    g.pull(bad.cuda())
+    assert g.status().code() == StatusCode.ERROR and g.size() == 500
+    g.reset()
+    same(g, c, old)
+    step(g, c, torch.arange(1548) * 13 + 2)             # all rows that are left, check() included
+    same(g, c, torch.cat([old, torch.arange(1548) * 13 + 2]))
