@@ -54,15 +54,16 @@ struct Slot4 {
     long long key;
     unsigned row, aux;
 };
-// One slot in one 16-byte access that does not allocate in L1 (other CTAs change the words behind our back). The words are
-// independent: each user re-checks what it needs with an atomic or after a barrier.
+// One slot in one 16-byte access that does not allocate in L1 (other CTAs change the words behind our back). Two 64-bit
+// elements, since each element of a vector access is single-copy atomic by itself: the key is read whole beside a 64-bit
+// CAS of another CTA. Row and aux may be older than it; each user re-checks what it needs with an atomic or after a barrier.
 __device__ __forceinline__ Slot4 ld_slot(const Slot* p) {
-    unsigned a, b, c, d;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "l"(p) : "memory");
+    unsigned long long key, rest;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0,%1}, [%2];" : "=l"(key), "=l"(rest) : "l"(p) : "memory");
     Slot4 s;
-    s.key = (long long)(((unsigned long long)b << 32) | a);
-    s.row = c;
-    s.aux = d;
+    s.key = (long long)key;
+    s.row = (unsigned)rest;
+    s.aux = (unsigned)(rest >> 32);
     return s;
 }
 
