@@ -359,13 +359,15 @@ Status SparseEngine::pull(const long long* keys, uint32_t n, uint32_t bag_size, 
         reserve = table_->reserve_rows(worst);
     }
     // One GPU: the local kernels; not for plans that the ordered sums or the replica log are made from, and not for a
-    // plan without insertion, whose missing keys only the general one can hold. A local plan puts arrays with an entry per
+    // plan without insertion, whose missing keys only the general one can hold. Without insertion and with no push
+    // announced it is a lookup; one that is followed by a push would have its keys deduplicated behind it (1 Mi keys of dim
+    // 64, pull and push: 571 us like that, 540 us when the pull makes the plan; 8192 keys of dim 16: 49 and 40 us). A local plan puts arrays with an entry per
     // position into the memory of the mailboxes, so a batch of more positions than those hold (pair_capacity) is the
     // general kernel's, which needs room for its distinct keys only and reports it when there is none.
     Plan kind = Plan::kGeneral;
     if (cfg_.world == 1 && n <= C_ && !deterministic_ && mirror_ == nullptr) {
         if (flags & FUSED_INSERT) kind = Plan::kLocal;
-        else if (flags & FUSED_COPY_ROWS) kind = Plan::kLookup;
+        else if ((flags & FUSED_COPY_ROWS) && !(flags & FUSED_PREPARE_PUSH)) kind = Plan::kLookup;
     }
     int rc;
     if (kind == Plan::kGeneral) {

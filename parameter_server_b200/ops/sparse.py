@@ -174,7 +174,7 @@ class SparseTable:
                 flags |= C.FUSED_OUT_BF16
             if insert:
                 flags |= C.FUSED_INSERT
-            if for_push:
+            if for_push and (insert or not self.read_only):   # a predictor's table: no push to prepare
                 flags |= C.FUSED_PREPARE_PUSH
             if mean:
                 flags |= C.FUSED_MEAN

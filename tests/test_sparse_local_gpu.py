@@ -109,6 +109,21 @@ def test_a_plan_of_another_kind_is_remade_for_the_push(how):
     same_tables(g, c, keys)
 
 
+@pytest.mark.parametrize("insert,for_push,launches", [(False, True, 2), (True, True, 2), (True, False, 2), (False, False, 3)])
+def test_a_pull_that_announces_a_push_leaves_its_plan(insert, for_push, launches):
+    """Pull and push are one launch each; only a lookup with no push announced is planned behind it when one comes."""
+    g, c = pair(32, "adagrad", 4096)
+    keys = batch(3000, [200, 33, 2], 8)
+    g.pull(keys.cuda()); c.pull(keys)
+    grads = whole(3000, 32, 9)
+    for _ in range(2):
+        before = g.engine.kernel_launches()
+        assert torch.equal(g.pull(keys.cuda(), insert=insert, for_push=for_push).cpu(), c.pull(keys))
+        g.push(grads.cuda()); c.push(grads)
+        assert g.engine.kernel_launches() - before == launches
+    same_tables(g, c, keys)
+
+
 @pytest.mark.parametrize("general", [False, True])
 def test_rows_erased_between_pull_and_push_get_nothing(general):
     g, c = pair(32, "sum", 4096)
