@@ -142,6 +142,29 @@ def test_rows_erased_between_pull_and_push_get_nothing(general):
     assert torch.allclose(rows.cpu()[kept], before.cpu()[kept] + count[kept][:, None], rtol=2.0 ** -22, atol=0)   # one rounding of the sum
 
 
+@pytest.mark.parametrize("dim,bags,bag,mean", [(4, 1, 1, False), (16, 1, 5000, False), (8, 3, 1025, False), (16, 64, 1024, True), (64, 1031, 1, False), (32, 257, 8, True),
+                                               (100, 77, 3, False), (128, 4099, 2, True), (256, 300, 1, False), (260, 33, 37, False)])
+@pytest.mark.parametrize("sms", [0, 3])
+def test_lookup_is_the_host_tables_pull(dim, bags, bag, mean, sms):
+    """Few large bags, many small ones, one in seven keys unknown; rows are whole numbers, so pooled sums are exact."""
+    n = bags * bag
+    g = pair(dim, "sum", n, read_only=True, init_range=0.0)[0]
+    c = SparseTable(dim, "sum", device="cpu", init_range=0.0)
+    if sms:
+        g.set_sm_budget(sms, sms)
+    keys = batch(n, [n // 5, 3], 11)
+    known = torch.unique(keys)
+    known = known[torch.arange(known.numel()) % 7 != 3]
+    rows = whole(known.numel(), dim, 12)
+    if known.numel():
+        g.set_rows(known.cuda(), rows.cuda(), emb_only=True); c.set_rows(known, rows, emb_only=True)
+    for dt in (torch.float32, torch.bfloat16)[:2 if dim % 8 == 0 else 1]:
+        out = g.pull(keys.cuda(), bag, mean, for_push=False, out_dtype=dt)
+        g.check()
+        assert torch.equal(out.cpu(), c.pull(keys, bag, mean, insert=False).to(dt))
+    assert g.size() == known.numel()
+
+
 def test_lookup_of_unknown_keys_probe_chains_and_a_push_that_drops_them():
     """A nearly full index (chains of several slots), erased entries on the chains, unknown keys among the known."""
     g = SparseTable(8, "sum", device="cuda", capacity=1024, max_keys=4096, max_rows=2048, slab_shift=11, init_range=0.0)
