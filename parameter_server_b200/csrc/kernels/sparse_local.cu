@@ -641,7 +641,9 @@ __device__ __forceinline__ void note_row(const TableView& T, KernelCtl* ctl, uns
 // 1 Mi keys of dim 64 (0.53 Mi distinct) with an Adagrad slot: 110 to 140 us for 830 MB, against 274 of the general kernel; the
 // rest of the way to 125 us at copy speed is the tail of the longest work items. A kernel per update rule: with the rule
 // looked up per coordinate the loops spill.
-template <int kThreads, int kOpt, bool kSync>
+// kFull: blocks of 32 positions (once_shift); with the shift in a register FTRL's push was 4 us longer at 512 Ki keys of
+// dim 32 and at 256 Ki of dim 64, the others up to 1 us.
+template <int kThreads, int kOpt, bool kSync, bool kFull>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_push_kernel(const LocalArgs a) {
     if (ld_acquire_gpu(&a.ctl->status) != 0u || ld_acquire_gpu(&a.plan_ctl->status) != 0u) return;
     const unsigned epoch = *((volatile unsigned*)&a.ctl->epoch) + 1u;
@@ -819,18 +821,19 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_push_kernel(c
     PROF(14);
     PROF(15);
     PROF_CTA(3);
-    // ---- keys that occur once: a warp takes 32 consecutive positions, its lane groups share the ones that qualify ---
+    // ---- keys that occur once: a warp takes a block of consecutive positions, its lane groups share the ones that qualify ---
     {
         // rows in flight per lane group: as many as the registers hold without spilling (a row is two to four 16-byte loads)
         constexpr int kIn = kOpt == OPT_FTRL || kOpt == OPT_ADAM || (kOpt < 0 && !kSync) ? 1 : 2;
         __shared__ uint2 s_todo[kThreads / 32][32];
         const unsigned warp = tid >> 5, nwarps = nthreads >> 5, gpw = 32u / lanes, g = wlane / lanes;
-        const unsigned nblk = (a.n + 31u) / 32u;
+        const unsigned sh = kFull ? 5u : a.once_shift;
+        const unsigned nblk = (a.n + (1u << sh) - 1u) >> sh;
         // Half of the blocks are dealt out by number, the rest from a counter to whoever is through with its work items, in
         // pieces that shrink towards the end (all of them dealt out left the CTAs with long items behind the others by half the
         // kernel's time; pieces of four to the end did the same to a batch of two blocks per warp).
         const unsigned fixed = max(1u, nblk / nwarps / 2u) * nwarps;
-        auto rows_of = [&](unsigned b) -> unsigned { return b < nblk && b * 32u + wlane < a.n ? a.push_row[b * 32u + wlane] : kDupRow; };
+        auto rows_of = [&](unsigned b) -> unsigned { return b < nblk && wlane >> sh == 0u && (b << sh) + wlane < a.n ? a.push_row[(b << sh) + wlane] : kDupRow; };
         unsigned at = warp, end = 0;   // the last block handed out; the end of the piece it is from
         auto next_block = [&]() -> unsigned {
             if (at + nwarps < fixed) return at += nwarps;
@@ -847,7 +850,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_push_kernel(c
         unsigned blk = warp;
         unsigned nxr = rows_of(blk);
         while (blk < nblk) {
-            const unsigned i0 = blk * 32u;
+            const unsigned i0 = blk << sh;
             unsigned row = nxr;
             blk = next_block();
             nxr = rows_of(blk);
@@ -990,19 +993,30 @@ __global__ void plan_finish_kernel(const LocalArgs a, const GeneralPlan g, unsig
     g.in_cnt[par * kMaxWorld] = n;
 }
 
-template <int kThreads>
+template <int kThreads, bool kFull>
 const void* push_kernel_of(int opt, bool sync) {
-    if (sync) return (const void*)local_push_kernel<kThreads, -1, true>;
+    if (sync) return (const void*)local_push_kernel<kThreads, -1, true, false>;
     switch (opt) {
-        case OPT_SGD: return (const void*)local_push_kernel<kThreads, OPT_SGD, false>;
-        case OPT_ADAGRAD: return (const void*)local_push_kernel<kThreads, OPT_ADAGRAD, false>;
-        case OPT_FTRL: return (const void*)local_push_kernel<kThreads, OPT_FTRL, false>;
-        case OPT_ADAM: return (const void*)local_push_kernel<kThreads, OPT_ADAM, false>;
-        default: return (const void*)local_push_kernel<kThreads, -1, false>;
+        case OPT_SGD: return (const void*)local_push_kernel<kThreads, OPT_SGD, false, kFull>;
+        case OPT_ADAGRAD: return (const void*)local_push_kernel<kThreads, OPT_ADAGRAD, false, kFull>;
+        case OPT_FTRL: return (const void*)local_push_kernel<kThreads, OPT_FTRL, false, kFull>;
+        case OPT_ADAM: return (const void*)local_push_kernel<kThreads, OPT_ADAM, false, kFull>;
+        default: return (const void*)local_push_kernel<kThreads, -1, false, false>;
     }
 }
 
 unsigned ceil_div(unsigned long long a, unsigned long long b) { return (unsigned)((a + b - 1) / b); }
+
+// Positions per block of the keys that occur once (its logarithm): 32, fewer while that leaves warps without a block, but not
+// fewer than the warp has lane groups. A wide row is a whole warp's work: 32 of them in a string took 41.2 us at 13312
+// distinct keys of dim 256 (most of 4736 warps idle; the general kernel 27.1), 15.4 us like this; dim 128, 26.1 and 14.8.
+// More blocks than one per warp cost more than their balance gives (65536 keys of dim 64, two: 19.4 to 23.0 us).
+unsigned once_shift(unsigned n, unsigned dim, unsigned warps) {
+    const unsigned groups = 32u / lanes_for_dim(dim);
+    unsigned sh = 5;
+    while ((1u << sh) > groups && n >> sh < warps) --sh;
+    return sh;
+}
 
 }  // namespace
 
@@ -1034,13 +1048,16 @@ int launch_local_pull(const LocalArgs& args, int max_blocks, bool wide, void* st
     return (int)cudaLaunchCooperativeKernel(k, dim3(grid), dim3(wide ? 1024 : 256), params, wide ? Tile<1024>::kSmem : Tile<256>::kSmem, (cudaStream_t)stream);
 }
 
-int launch_local_push(const LocalArgs& a, int max_blocks, bool wide, bool sync, unsigned table_slots, void* stream) {
+int launch_local_push(const LocalArgs& args, int max_blocks, bool wide, bool sync, unsigned table_slots, void* stream) {
+    LocalArgs a = args;
     void* params[] = {(void*)&a};
     const int opt = (unsigned)opt_num_slots(a.opt.type) == table_slots ? a.opt.type : -1;
-    const void* k = wide ? push_kernel_of<1024>(opt, sync) : push_kernel_of<256>(opt, sync);
     const unsigned threads = wide ? 1024 : 256;
     const unsigned want = ceil_div((unsigned long long)a.n * lanes_for_dim(a.dim), threads);
     const unsigned grid = want < 1 ? 1 : (want < (unsigned)max_blocks ? want : (unsigned)max_blocks);
+    a.once_shift = once_shift(a.n, a.dim, grid * (threads / 32));
+    const void* k = a.once_shift == 5 ? (wide ? push_kernel_of<1024, true>(opt, sync) : push_kernel_of<256, true>(opt, sync))
+                                      : (wide ? push_kernel_of<1024, false>(opt, sync) : push_kernel_of<256, false>(opt, sync));
     return (int)cudaLaunchKernel(k, dim3(grid), dim3(threads), params, 0, (cudaStream_t)stream);
 }
 

@@ -8,6 +8,7 @@ struct LocalArgs {
     unsigned n, bag_size, dim, flags;
     unsigned item_len, big_min, big_len;   // occurrences per work item of a lane group; a key with more than big_min is cut into
                                            // CTA items of big_len (set by launch_local_pull)
+    unsigned once_shift;         // push: a block of keys that occur once has 1 << once_shift positions (set by launch_local_push)
     const long long* keys;       // [n]
     void* out;                   // [n / bag_size][dim] fp32, or bf16 with FUSED_OUT_BF16
     const float* grads;          // [n / bag_size][dim]

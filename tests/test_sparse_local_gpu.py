@@ -63,6 +63,21 @@ def test_step_is_the_host_tables_step(dim, opt, n, hot, sms):
         assert torch.equal(g.pull(keys.cuda(), insert=False, out_dtype=torch.bfloat16).cpu(), c.pull(keys).bfloat16())
 
 
+# once-only keys of wide rows, from one position per block to thirty-two (148 SMs hold 4736 warps, a budget of 5 holds 160)
+@pytest.mark.parametrize("dim,opt,n", [(256, "ftrl", 4735), (256, "adagrad", 9473), (128, "adam", 13312), (128, "sgd", 37889), (100, "ftrl", 75777), (256, "sum", 151553)])
+@pytest.mark.parametrize("sms", [0, 5])
+def test_keys_that_occur_once_at_every_block_length(dim, opt, n, sms):
+    g, c = pair(dim, opt, n)
+    if sms:
+        g.set_sm_budget(sms, sms)
+    keys = batch(n, [2], n)
+    grads = whole(n, dim, 5)
+    for _ in range(2):
+        g.pull(keys.cuda()); c.pull(keys)
+        g.push(grads.cuda()); c.push(grads)
+    same_tables(g, c, keys)
+
+
 @pytest.mark.parametrize("bag,mean", [(2, False), (4, True), (8, True)])
 def test_pooled_step(bag, mean):
     g, c = pair(32, "sgd", 4096)
