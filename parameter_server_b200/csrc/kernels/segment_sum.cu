@@ -12,7 +12,8 @@ namespace {
 
 constexpr int kThreads = 256;
 
-__global__ void iota_kernel(unsigned* p, unsigned n) {
+__global__ void iota_kernel(unsigned* p, unsigned n, unsigned* long_cnt) {
+    if (blockIdx.x == 0 && threadIdx.x < 2) long_cnt[threadIdx.x] = 0;
     for (unsigned i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) p[i] = i;
 }
 
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(kThreads) ordered_sum_kernel(const unsigned* _
                                                               const unsigned* __restrict__ sorted_pos, unsigned n, const PlanWords plan,
                                                               const float* __restrict__ grads, unsigned bag, unsigned dim,
                                                               float scale, float* __restrict__ agg, unsigned* __restrict__ long_cnt,
-                                                              uint4* __restrict__ long_runs, uint2* __restrict__ blocks, unsigned max_blocks) {
+                                                              uint4* __restrict__ long_runs, uint4* __restrict__ blocks, unsigned max_blocks) {
     if (plan.cut_short()) return;
     const unsigned lanes = lanes_for_dim(dim);
     const unsigned tid = blockIdx.x * kThreads + threadIdx.x;
@@ -99,16 +100,20 @@ __global__ void __launch_bounds__(kThreads) ordered_sum_kernel(const unsigned* _
         if (lo >= end || end > n) continue;   // an id without a run: nothing below may leave the arrays for it
         if (end - lo > kBlock) {
             const unsigned nblk = (end - lo + kBlock - 1) / kBlock;
-            unsigned base = 0;
+            unsigned base = 0, run = 0;
             if (lane == 0) {
                 base = atomicAdd(long_cnt + 1, nblk);   // work items, and rows of the scratch area for their sums
-                if (base + nblk <= max_blocks) long_runs[atomicAdd(long_cnt, 1u)] = make_uint4(u, base, nblk, 0u);
+                if (base + nblk <= max_blocks) {
+                    run = atomicAdd(long_cnt, 1u);
+                    long_runs[run] = make_uint4(u, base, nblk, 0u);
+                }
             }
             const unsigned wl = threadIdx.x & 31u, gl0 = wl / lanes * lanes;
             const unsigned gmask = (lanes >= 32u ? 0xffffffffu : ((1u << lanes) - 1u)) << gl0;
             base = __shfl_sync(gmask, base, gl0);
+            run = __shfl_sync(gmask, run, gl0);
             if (base + nblk > max_blocks) continue;
-            for (unsigned k = lane; k < nblk; k += lanes) blocks[base + k] = make_uint2(lo + k * kBlock, min(end, lo + (k + 1) * kBlock));
+            for (unsigned k = lane; k < nblk; k += lanes) blocks[base + k] = make_uint4(lo + k * kBlock, min(end, lo + (k + 1) * kBlock), run, 0u);
             continue;
         }
         for (unsigned d = lane * 4; d < dim; d += lanes * 4)
@@ -116,45 +121,46 @@ __global__ void __launch_bounds__(kThreads) ordered_sum_kernel(const unsigned* _
     }
 }
 
-// Pass 3, one lane group per block of a long run.
+// The block sums of a long run, front to back. The adds are chained; sixteen loads at a time are not.
+__device__ __forceinline__ float4 fold(const float* part, unsigned n, unsigned dim) {
+    constexpr unsigned kIn = 16;
+    float4 acc = __ldcg((const float4*)part);
+    unsigned k = 1;
+    for (; k + kIn <= n; k += kIn) {
+        float4 v[kIn];
+#pragma unroll
+        for (unsigned t = 0; t < kIn; ++t) v[t] = __ldcg((const float4*)(part + (size_t)(k + t) * dim));
+#pragma unroll
+        for (unsigned t = 0; t < kIn; ++t) add_rn(acc, v[t]);
+    }
+    for (; k < n; ++k) add_rn(acc, __ldcg((const float4*)(part + (size_t)k * dim)));
+    return acc;
+}
+
+// Pass 3, one lane group per block of a long run; the group that stores the last block sum of a run folds them. (The folds in a
+// launch of their own, and a memset of the two counters, cost a batch of 256 to 8192 keys 3 to 11 % of its step.)
 __global__ void __launch_bounds__(kThreads) block_sum_kernel(const unsigned* __restrict__ sorted_pos, unsigned n, const float* __restrict__ grads,
                                                             unsigned bag, unsigned dim, float scale, const unsigned* __restrict__ long_cnt,
-                                                            const uint2* __restrict__ blocks, unsigned max_blocks, float* __restrict__ partials) {
+                                                            uint4* long_runs, const uint4* __restrict__ blocks, unsigned max_blocks,
+                                                            float* partials, float* __restrict__ agg) {
     const unsigned lanes = lanes_for_dim(dim);
     const unsigned tid = blockIdx.x * kThreads + threadIdx.x;
     const unsigned n_blocks = min(long_cnt[1], max_blocks), lane = tid % lanes;
+    const unsigned gl0 = (threadIdx.x & 31u) / lanes * lanes, gmask = (lanes >= 32u ? 0xffffffffu : ((1u << lanes) - 1u)) << gl0;
     for (unsigned k = tid / lanes; k < n_blocks; k += (gridDim.x * kThreads) / lanes) {
-        const uint2 b = blocks[k];
-        if (b.x >= b.y || b.y > n) continue;
+        const uint4 b = blocks[k];
+        if (b.x >= b.y || b.y > n || b.z >= max_blocks / 2) continue;
         for (unsigned d = lane * 4; d < dim; d += lanes * 4)
             *(float4*)(partials + (size_t)k * dim + d) = run_sum(sorted_pos, b.x, b.y, grads, bag, dim, d, scale);
-    }
-}
-
-// Pass 4, one lane group per long run: the block sums front to back. The adds are chained; sixteen loads at a time are not.
-__global__ void __launch_bounds__(kThreads) fold_blocks_kernel(unsigned dim, const unsigned* __restrict__ long_cnt,
-                                                              const uint4* __restrict__ long_runs, const float* __restrict__ partials,
-                                                              float* __restrict__ agg) {
-    constexpr unsigned kIn = 16;
-    const unsigned lanes = lanes_for_dim(dim);
-    const unsigned tid = blockIdx.x * kThreads + threadIdx.x;
-    const unsigned n_long = long_cnt[0], lane = tid % lanes;
-    for (unsigned r = tid / lanes; r < n_long; r += (gridDim.x * kThreads) / lanes) {
-        const uint4 run = long_runs[r];
-        const float* part = partials + (size_t)run.y * dim;
-        for (unsigned d = lane * 4; d < dim; d += lanes * 4) {
-            float4 acc = *(const float4*)(part + d);
-            unsigned k = 1;
-            for (; k + kIn <= run.z; k += kIn) {
-                float4 v[kIn];
-#pragma unroll
-                for (unsigned t = 0; t < kIn; ++t) v[t] = *(const float4*)(part + (size_t)(k + t) * dim + d);
-#pragma unroll
-                for (unsigned t = 0; t < kIn; ++t) add_rn(acc, v[t]);
-            }
-            for (; k < run.z; ++k) add_rn(acc, *(const float4*)(part + (size_t)k * dim + d));
-            *(float4*)(agg + (size_t)run.x * dim + d) = acc;
-        }
+        __threadfence();
+        __syncwarp(gmask);
+        const uint4 run = __ldcg(long_runs + b.z);   // (its last word changes meanwhile)
+        unsigned stored = 0;
+        if (lane == 0) stored = atomicAdd(&long_runs[b.z].w, 1u) + 1u;
+        if (__shfl_sync(gmask, stored, gl0) != run.z) continue;
+        __threadfence();
+        for (unsigned d = lane * 4; d < dim; d += lanes * 4)
+            *(float4*)(agg + (size_t)run.x * dim + d) = fold(partials + (size_t)run.y * dim + d, run.z, dim);
     }
 }
 
@@ -175,7 +181,7 @@ Scratch scratch_layout(unsigned max_n, unsigned dim, size_t cub_bytes) {
     l.starts = o; o += up(((size_t)max_n + 1) * sizeof(unsigned));
     l.runs = o; o += up(max_long * sizeof(uint4));
     l.max_blocks = (unsigned)(2 * max_long + 1);                        // sum of ceil(len / kBlock) over the long runs
-    l.blocks = o; o += up(l.max_blocks * sizeof(uint2));
+    l.blocks = o; o += up(l.max_blocks * sizeof(uint4));
     l.partials = o; o += up(l.max_blocks * (size_t)dim * sizeof(float));
     l.total = o;
     return l;
@@ -204,16 +210,14 @@ int ordered_segment_sum(const int* inverse, unsigned n, unsigned max_n, const un
     unsigned* long_cnt = (unsigned*)((char*)temp + l.counters);
     unsigned* starts = (unsigned*)((char*)temp + l.starts);
     uint4* long_runs = (uint4*)((char*)temp + l.runs);
-    uint2* blocks = (uint2*)((char*)temp + l.blocks);
+    uint4* blocks = (uint4*)((char*)temp + l.blocks);
     float* partials = (float*)((char*)temp + l.partials);
     const PlanWords plan = {counters, pull_ctl, push_ctl};
-    cudaError_t e = cudaMemsetAsync(long_cnt, 0, 8, s);
-    if (e != cudaSuccess) return (int)e;
-    iota_kernel<<<148 * 2, kThreads, 0, s>>>(iota, n);
+    iota_kernel<<<148 * 2, kThreads, 0, s>>>(iota, n, long_cnt);
     int bits = 1;
     while (bits < 31 && (1ull << bits) < (unsigned long long)n) ++bits;   // unique ids are below n; bit 31 is a flag, not part of the id
     size_t cb = cub_bytes;
-    e = cub::DeviceRadixSort::SortPairs(cub_temp, cb, (const unsigned*)inverse, sorted_ids, (const unsigned*)iota, sorted_pos, (int)n, 0,
+    const cudaError_t e = cub::DeviceRadixSort::SortPairs(cub_temp, cb, (const unsigned*)inverse, sorted_ids, (const unsigned*)iota, sorted_pos, (int)n, 0,
                                         bits, s);
     if (e != cudaSuccess) return (int)e;
     const unsigned lanes = lanes_for_dim(dim);
@@ -224,10 +228,8 @@ int ordered_segment_sum(const int* inverse, unsigned n, unsigned max_n, const un
     ordered_sum_kernel<<<grid, kThreads, 0, s>>>(starts, sorted_pos, n, plan, grads, bag, dim, scale, agg, long_cnt, long_runs, blocks, l.max_blocks);
     // at most n / kBlock + (long runs) blocks, and a long run has more than kBlock entries
     const unsigned long long want_blocks = (2ull * n / kBlock * lanes + kThreads - 1) / kThreads + 1;
-    block_sum_kernel<<<(unsigned)(want_blocks < 148 * 8 ? want_blocks : 148 * 8), kThreads, 0, s>>>(sorted_pos, n, grads, bag, dim, scale, long_cnt, blocks, l.max_blocks,
-                                                                                                             partials);
-    const unsigned long long want_runs = ((unsigned long long)n / kBlock * lanes + kThreads - 1) / kThreads + 1;
-    fold_blocks_kernel<<<(unsigned)(want_runs < 148 * 2 ? want_runs : 148 * 2), kThreads, 0, s>>>(dim, long_cnt, long_runs, partials, agg);
+    block_sum_kernel<<<(unsigned)(want_blocks < 148 * 8 ? want_blocks : 148 * 8), kThreads, 0, s>>>(sorted_pos, n, grads, bag, dim, scale, long_cnt, long_runs, blocks,
+                                                                                                             l.max_blocks, partials, agg);
     return (int)cudaGetLastError();
 }
 
