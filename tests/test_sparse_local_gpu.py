@@ -40,7 +40,8 @@ def batch(n, hot, seed):
     return k[torch.randperm(n, generator=torch.Generator().manual_seed(seed))]
 
 
-# a work item holds 32 occurrences, a tile 1024 (2048) keys, a warp 32 positions; lane groups of 1 .. 32 lanes
+# below 2^18 keys a work item of a lane group holds 16 occurrences and a key of more than 1024 goes to CTA items of 256; a tile
+# holds 1024 (2048) keys; lane groups of 1 .. 32 lanes
 @pytest.mark.parametrize("dim,opt,n,hot", [
     (4, "sum", 1, []), (4, "sgd", 31, [2]), (8, "adagrad", 33, [31, 2]), (16, "adagrad", 257, [32, 33]), (64, "adagrad", 1025, [64, 65, 2, 3]),
     (64, "ftrl", 4099, [33, 1000]), (100, "adam", 3001, [2, 2, 2, 500]), (32, "sum", 9001, [1025, 1024, 2048, 2049, 3]), (128, "adagrad", 70001, [40000, 97, 32, 31]), (256, "sgd", 2049, [1500, 2]),
@@ -76,6 +77,30 @@ def test_keys_that_occur_once_at_every_block_length(dim, opt, n, sms):
         g.pull(keys.cuda()); c.pull(keys)
         g.push(grads.cuda()); c.push(grads)
     same_tables(g, c, keys)
+
+
+# The three ways a batch's repeated keys are cut into work items: lane-group items of 16 occurrences and CTA items of 256 above 1024
+# (below 2^18 keys), 32 and 512 above 2048 (below 2^21), 32 and 1024 above 2048. 700 001 keys are several tiles per CTA.
+CUTS = {(1 << 18) - 1: [15, 16, 17, 31, 32, 33, 255, 256, 257, 1023, 1024, 1025, 1279, 1280, 1281, 5000],
+        1 << 18: [15, 17, 31, 32, 33, 63, 64, 65, 1025, 2047, 2048, 2049, 2559, 2560, 2561, 20000],
+        700001: [32, 33, 2048, 2049, 4607, 4608, 4609, 150000],
+        (1 << 21) - 1: [33, 2048, 2049, 3071, 3072, 3073, 200000],
+        1 << 21: [32, 33, 64, 65, 2048, 2049, 3071, 3072, 3073, 4097, 300000]}
+
+
+@pytest.mark.parametrize("dim,opt,n,sms", [(4, "sum", (1 << 18) - 1, 0), (4, "sum", 1 << 18, 0), (64, "adagrad", (1 << 18) - 1, 0), (64, "adagrad", 1 << 18, 7), (16, "ftrl", 1 << 18, 0),
+                                           (4, "sum", 700001, 0), (16, "adagrad", 700001, 0), (4, "sum", (1 << 21) - 1, 0), (4, "sum", 1 << 21, 0), (8, "adagrad", 1 << 21, 148)])
+def test_step_of_large_batches_at_the_edges_of_their_work_items(dim, opt, n, sms):
+    g, c = pair(dim, opt, n)
+    if sms:
+        g.set_sm_budget(sms, sms)
+    keys = batch(n, CUTS[n], n)
+    grads = whole(n, dim, 1)
+    for _ in range(2):
+        g.pull(keys.cuda()); c.pull(keys)
+        g.push(grads.cuda()); c.push(grads)
+    same_tables(g, c, keys)
+    assert torch.equal(g.pull(keys.cuda()).cpu(), c.pull(keys))
 
 
 @pytest.mark.parametrize("bag,mean", [(2, False), (4, True), (8, True)])
