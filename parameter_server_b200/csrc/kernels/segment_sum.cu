@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kThreads) run_starts_kernel(const unsigned* __
 // Pass 2, one lane group per unique id u: a run of up to kBlock entries is summed here; a longer one gets a row of
 // partial sums and a work item per block, on which the whole GPU works in pass 3. One CTA per long run left the hottest
 // key's 20 000 occurrences of a 213 Ki batch of dim 128 to eight lane groups, and two binary searches per key (36 dependent
-// loads) came before: a step of 763 us, 285 us with these passes. What bounds them now is the latency of short kernels.
+// loads) came before: a step of 763 us, 267 us with these passes. What bounds them now is the latency of short kernels.
 __global__ void __launch_bounds__(kThreads) ordered_sum_kernel(const unsigned* __restrict__ starts,
                                                               const unsigned* __restrict__ sorted_pos, unsigned n, const PlanWords plan,
                                                               const float* __restrict__ grads, unsigned bag, unsigned dim,

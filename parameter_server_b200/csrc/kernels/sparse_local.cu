@@ -36,7 +36,14 @@ namespace {
 // row per 32 occurrences the hottest key of 4 Mi Zipf(1.05) keys (210 000 of them) took 548 us. So a key with more than
 // big_min is summed by whole CTAs, big_len occurrences each. Those items are a string of memory latencies and CTA
 // barriers (eight rows requested at a time), up to 10 us each even when short (with big_min 128 the five hundred of a 213 Ki batch took 50 of the
-// push's 78 us on 96 SMs): few of them, and no longer than the batch allows.
+// push's 78 us on 96 SMs): few of them, and no longer than the batch allows. By the batch's size alone: the cost is that of the
+// longest item against the push's time. Pull and push in us with the first / second / third cut for all sizes, Adagrad:
+//   dim 64, Zipf 1.05      64 Ki 57.2 / 58.4 / 59.7   256 Ki 110 / 113 / 115   1 Mi 292 / 292 / 289   4 Mi 969 / 946 / 950
+//   dim 16, Zipf 1.1       64 Ki 54.6 / 53.8 / 54.3   256 Ki  71 /  71 /  72   1 Mi 200 / 187 / 185   4 Mi 682 / 611 / 608
+//   dim 128, Zipf 1.1      64 Ki 70.4 / 70.1 / 77.6   256 Ki 146 / 150 / 159   1 Mi 412 / 410 / 409   2 Mi 761 / 752 / 748
+//   dim 128 on 96 SMs      64 Ki 70.7 / 72.4 / 72.1   256 Ki 162 / 159 / 156   1 Mi 512 / 475 / 465   2 Mi 984 / 892 / 865
+// Where two cuts cross depends on dim and SMs (first and second: near 2^17 keys at dim 16, 2^19 at dim 128 on all SMs), but
+// these lines cost nowhere more than 3 us or 5 %.
 struct Cut {
     unsigned item_len, big_min, big_len;
 };
@@ -639,8 +646,8 @@ __device__ __forceinline__ void note_row(const TableView& T, KernelCtl* ctl, uns
 }
 
 // 1 Mi keys of dim 64 (0.53 Mi distinct) with an Adagrad slot: 110 to 140 us for 830 MB, against 274 of the general kernel; the
-// rest of the way to 125 us at copy speed is the tail of the longest work items. A kernel per update rule: with the rule
-// looked up per coordinate the loops spill.
+// rest of the way to 125 us at copy speed is the tail of the longest work items. A kernel per update rule: at 64 registers the
+// loops spill 268 bytes a thread with the rule looked up per coordinate, 20 with sgd, 24 Adagrad, 104 Adam, 116 FTRL.
 // kFull: blocks of 32 positions (once_shift); with the shift in a register FTRL's push was 4 us longer at 512 Ki keys of
 // dim 32 and at 256 Ki of dim 64, the others up to 1 us.
 template <int kThreads, int kOpt, bool kSync, bool kFull>
@@ -823,7 +830,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_push_kernel(c
     PROF_CTA(3);
     // ---- keys that occur once: a warp takes a block of consecutive positions, its lane groups share the ones that qualify ---
     {
-        // rows in flight per lane group: as many as the registers hold without spilling (a row is two to four 16-byte loads)
+        // rows in flight per lane group: two where a row and its slots are at most three 16-byte loads a thread, else one (the
+        // kernels spill a few values either way)
         constexpr int kIn = kOpt == OPT_FTRL || kOpt == OPT_ADAM || (kOpt < 0 && !kSync) ? 1 : 2;
         __shared__ uint2 s_todo[kThreads / 32][32];
         const unsigned warp = tid >> 5, nwarps = nthreads >> 5, gpw = 32u / lanes, g = wlane / lanes;

@@ -37,7 +37,7 @@ struct LocalArgs {
     unsigned* occ;               // [N] positions of the repeated keys, one contiguous segment per key (phase A: slots of
                                  //     the keys that this call inserted)
     uint4* items;                // [N/2] {row, first occurrence, length | items of the key << 8, 1 + hot index or 0}
-    uint4* big_items;            // [N/128 + 1] the same for keys that whole CTAs sum (length | items << 11)
+    uint4* big_items;            // [2 (N/256) + 1] the same for keys that whole CTAs sum (length | items << 11)
     long long* key_copy;         // [N] lookup: the keys, in case a push follows
     float* hot_sum;              // [N/16 + 1][dim] sums of keys with several items: zero between calls
     unsigned* hot_cnt;           // [N/16 + 1] items of the key that have arrived: zero between calls

@@ -48,6 +48,7 @@ class SparseTable:
         max_keys: largest number of key positions in one pull / push call on this rank.
         n_shards: global shard count G (default: world size); keys map to shards with
             ``jump_consistent_hash(murmur(key), G)`` and shards to ranks with ``shard_owner``.
+        pair_capacity: distinct keys that one rank may send to one owner in a call (0 = automatic); more are an error status.
         sync: allocate the per-row delta section needed by ``sync_push`` + ``store``.
         replicate: allocate the replica log, so that pushes can keep a mirror on the next rank exact
             (``parallel.ReplicaSet(table, in_push=True)``).
@@ -155,7 +156,8 @@ class SparseTable:
              out: Optional[torch.Tensor] = None, for_push: bool = True, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         """Rows (sum/mean pooled over ``bag_size`` consecutive keys) of ``keys``; missing keys are
         inserted with their initial value unless the table is read-only. ``out`` (or ``out_dtype``) may be
-        bfloat16: the table stays fp32, the rows are rounded where they are read."""
+        bfloat16: the table stays fp32, the rows are rounded where they are read. ``for_push=False`` says that no push
+        follows (one that does is still right, but has its keys deduplicated first)."""
         insert = (not self.read_only) if insert is None else insert
         keys = keys.reshape(-1)
         n = keys.numel()
