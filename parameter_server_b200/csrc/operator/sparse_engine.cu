@@ -342,6 +342,11 @@ Status SparseEngine::make_general_plan(void* stream) {
     return Status::Ok();
 }
 
+namespace {
+// a pull without insertion that announces a push
+bool lookup_sort(unsigned flags) { return (flags & FUSED_PREPARE_PUSH) && !(flags & FUSED_INSERT); }
+}  // namespace
+
 Status SparseEngine::pull(const long long* keys, uint32_t n, uint32_t bag_size, void* out, unsigned flags,
                           void* stream) {
     if (failed_) return Status::Error("pull: the engine saw a fatal device status; call reset() on every rank first");
@@ -358,16 +363,18 @@ Status SparseEngine::pull(const long long* keys, uint32_t n, uint32_t bag_size, 
         if (!grown.ok() && grown.code() != StatusCode::OUT_OF_MEMORY) return grown;
         reserve = table_->reserve_rows(worst);
     }
-    // One GPU: the local kernels; not for plans that the ordered sums or the replica log are made from, and not for a
-    // plan without insertion, whose missing keys only the general one can hold. Without insertion and with no push
-    // announced it is a lookup; one that is followed by a push would have its keys deduplicated behind it (1 Mi keys of dim
-    // 64, pull and push: 571 us like that, 540 us when the pull makes the plan; 8192 keys of dim 16: 49 and 40 us). A local plan puts arrays with an entry per
-    // position into the memory of the mailboxes, so a batch of more positions than those hold (pair_capacity) is the
-    // general kernel's, which needs room for its distinct keys only and reports it when there is none.
+    // One GPU: the local kernels; not for plans that the ordered sums or the replica log are made from. A local plan puts
+    // arrays with an entry per position into the memory of the mailboxes, so a batch of more positions than those hold
+    // (pair_capacity) is the general kernel's, which needs room for its distinct keys only and reports it when there is none.
+    // A pull without insertion is a lookup (the missing keys of a plan only the general kernel can hold), and when a push
+    // follows, its keys are deduplicated behind it: 571 us for both at 1 Mi keys of dim 64, 540 when the pull makes the plan (49
+    // and 40 at 8192 keys of dim 16); with no push the pull alone is 192 and, as a lookup, 84 us (25 and 11). So a pull that
+    // announces a push makes the plan if the last plan of its sort was pushed. The rows are the same either way.
+    if (plan_valid_ && lookup_sort(plan_flags_)) lookups_pushed_ = plan_pushed_;
     Plan kind = Plan::kGeneral;
     if (cfg_.world == 1 && n <= C_ && !deterministic_ && mirror_ == nullptr) {
         if (flags & FUSED_INSERT) kind = Plan::kLocal;
-        else if ((flags & FUSED_COPY_ROWS) && !(flags & FUSED_PREPARE_PUSH)) kind = Plan::kLookup;
+        else if ((flags & FUSED_COPY_ROWS) && !(lookups_pushed_ && lookup_sort(flags))) kind = Plan::kLookup;
     }
     int rc;
     if (kind == Plan::kGeneral) {
@@ -392,7 +399,7 @@ Status SparseEngine::pull(const long long* keys, uint32_t n, uint32_t bag_size, 
     plan_bag_ = bag_size;
     plan_flags_ = flags;
     plan_valid_ = true;
-    plan_used_ = false;
+    plan_used_ = plan_pushed_ = false;
     if (!reserve.ok() && reserve.code() != StatusCode::OUT_OF_MEMORY) return reserve;
     return Status::Ok();
 }
@@ -404,6 +411,7 @@ Status SparseEngine::push(const float* grads, uint32_t n_rows, const OptConfig& 
         return Status::InvalidConfig("push: gradient rows (" + std::to_string(n_rows) + ") != pulled bags (" +
                                      std::to_string(plan_n_ / plan_bag_) + ")");
     cudaSetDevice(table_->device());
+    plan_pushed_ = true;
     if (plan_kind_ == Plan::kLocal && !deterministic_ && mirror_ == nullptr && !(flags & FUSED_AGG_READY)) {
         LocalArgs a;
         fill_local(a);

@@ -134,7 +134,7 @@ private:
     size_t sort_temp_bytes_ = 0;
     // last pull (the plan)
     // Which plan the last pull left. One GPU: a pull that inserts leaves a local plan, one that does not a lookup (its
-    // keys only); with reproducible pushes or a mirror, and with several ranks, the general one. A push that finds
+    // keys only) unless a push is to be expected; with reproducible pushes or a mirror, and with several ranks, the general one. A push that finds
     // another plan than the one it needs has it made first (make_general_plan).
     enum class Plan { kGeneral, kLocal, kLookup };
     Plan plan_kind_ = Plan::kGeneral;
@@ -145,7 +145,8 @@ private:
     const long long* plan_keys_ = nullptr;
     uint32_t plan_n_ = 0, plan_bag_ = 1;
     unsigned plan_flags_ = 0;
-    bool plan_valid_ = false, plan_used_ = false;
+    bool plan_valid_ = false, plan_used_ = false, plan_pushed_ = false;
+    bool lookups_pushed_ = false;   // the last plan of a pull without insertion that announced a push was pushed
     uint64_t launches_ = 0;
     unsigned long long* prof_ = nullptr;
     bool profile_ = false;

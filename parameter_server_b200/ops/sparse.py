@@ -157,7 +157,7 @@ class SparseTable:
         """Rows (sum/mean pooled over ``bag_size`` consecutive keys) of ``keys``; missing keys are
         inserted with their initial value unless the table is read-only. ``out`` (or ``out_dtype``) may be
         bfloat16: the table stays fp32, the rows are rounded where they are read. ``for_push=False`` says that no push
-        follows (one that does is still right, but has its keys deduplicated first)."""
+        follows (one that does is still right, but may have its keys deduplicated first)."""
         insert = (not self.read_only) if insert is None else insert
         keys = keys.reshape(-1)
         n = keys.numel()
@@ -176,7 +176,7 @@ class SparseTable:
                 flags |= C.FUSED_OUT_BF16
             if insert:
                 flags |= C.FUSED_INSERT
-            if for_push and (insert or not self.read_only):   # a predictor's table: no push to prepare
+            if for_push:
                 flags |= C.FUSED_PREPARE_PUSH
             if mean:
                 flags |= C.FUSED_MEAN

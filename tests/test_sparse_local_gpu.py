@@ -149,18 +149,40 @@ def test_a_plan_of_another_kind_is_remade_for_the_push(how):
     same_tables(g, c, keys)
 
 
-@pytest.mark.parametrize("insert,for_push,launches", [(False, True, 2), (True, True, 2), (True, False, 2), (False, False, 3)])
-def test_a_pull_that_announces_a_push_leaves_its_plan(insert, for_push, launches):
-    """Pull and push are one launch each; only a lookup with no push announced is planned behind it when one comes."""
+@pytest.mark.parametrize("insert,for_push,launches", [(False, True, [3, 2, 2]), (True, True, [2, 2]), (True, False, [2, 2]), (False, False, [3, 3])])
+def test_a_pull_that_a_push_is_expected_behind_leaves_its_plan(insert, for_push, launches):
+    """Pull and push are one launch each. A lookup is planned behind it when a push comes; the next pull that announces one expects it."""
     g, c = pair(32, "adagrad", 4096)
     keys = batch(3000, [200, 33, 2], 8)
     g.pull(keys.cuda()); c.pull(keys)
     grads = whole(3000, 32, 9)
-    for _ in range(2):
+    for want in launches:
         before = g.engine.kernel_launches()
         assert torch.equal(g.pull(keys.cuda(), insert=insert, for_push=for_push).cpu(), c.pull(keys))
         g.push(grads.cuda()); c.push(grads)
-        assert g.engine.kernel_launches() - before == launches
+        assert g.engine.kernel_launches() - before == want
+    same_tables(g, c, keys)
+
+
+def test_pulls_without_a_push_are_lookups_again():
+    g, c = pair(32, "adagrad", 4096)
+    keys = batch(3000, [200, 33, 2], 8)
+    grads = whole(3000, 32, 9)
+    g.pull(keys.cuda()); c.pull(keys)
+
+    def planned():      # how many launches it takes to know the number of distinct keys
+        assert torch.equal(g.pull(keys.cuda(), insert=False).cpu(), c.pull(keys))
+        before = g.engine.kernel_launches()
+        assert g.engine.last_unique(0) == torch.unique(keys).numel()
+        return g.engine.kernel_launches() - before
+
+    assert planned() == 1
+    g.push(grads.cuda()); c.push(grads)
+    assert planned() == 0 and planned() == 1 and planned() == 1
+    g.push(grads.cuda()); c.push(grads)
+    g.pull(keys.cuda()); c.pull(keys)                # of another sort: nothing to learn from
+    assert planned() == 0 and planned() == 1
+    g.push(grads.cuda()); c.push(grads)
     same_tables(g, c, keys)
 
 
