@@ -656,7 +656,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_push_kernel(c
     const unsigned epoch = *((volatile unsigned*)&a.ctl->epoch) + 1u;
     const unsigned* cnt = a.counters + (*((volatile const unsigned*)&a.plan_ctl->epoch) & 1u) * 16;
     const TableView T = *a.table;
-    // rows were erased since the plan was made: ask the slots again (an erased key's gradient is dropped)
+    // rows were erased since the plan was made: ask the slots again (an erased key's gradient is dropped). A key that found
+    // the pool exhausted is asked for in any case: it may have been given a row since.
     const bool stale = *((volatile unsigned*)T.erase_gen) != *((volatile unsigned*)a.plan_gen);
     // only Adam's rule changes with the call number; the others read their options where the parameters lie
     OptConfig stepped;
@@ -690,7 +691,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_push_kernel(c
             const unsigned len = it.z & 2047u, n_parts = it.z >> 11;
             const unsigned* occ = a.occ + it.y;
             unsigned row = it.x;
-            if (stale) row = T.slots[a.slot_of_id[a.id_of[occ[0]]]].row;
+            if (stale || row == kNoRow) row = T.slots[a.slot_of_id[a.id_of[occ[0]]]].row;
             if (row >= kRowPending) {
                 if (threadIdx.x == 0) set_soft_status(a.ctl, kStOom, W_NOROW);
                 continue;
@@ -772,7 +773,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_push_kernel(c
         if (e + ngroups < n_items) nx = a.items[e + ngroups];
         const unsigned len = cur.z & 255u;
         unsigned row = cur.x;
-        if (stale) row = T.slots[a.slot_of_id[a.id_of[p[0]]]].row;
+        if (stale || row == kNoRow) row = T.slots[a.slot_of_id[a.id_of[p[0]]]].row;
         if (row >= kRowPending) {
             if (lane == 0) set_soft_status(a.ctl, kStOom, W_NOROW);
             batch_of(nx, 0);
@@ -862,7 +863,10 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_push_kernel(c
             unsigned row = nxr;
             blk = next_block();
             nxr = rows_of(blk);
-            if (stale && row != kDupRow && row != kNoRow) row = T.slots[a.slot_of_id[a.id_of[i0 + wlane]]].row;
+            if (row != kDupRow && (stale || row == kNoRow)) {
+                const unsigned id = a.id_of[i0 + wlane];
+                if (id != kNoSlot) row = T.slots[a.slot_of_id[id]].row;
+            }
             if (row == kNoRow || row == kRowPending) {
                 set_soft_status(a.ctl, kStOom, W_NOROW);
                 row = kDupRow;

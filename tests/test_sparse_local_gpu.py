@@ -227,6 +227,28 @@ def test_lookup_is_the_host_tables_pull(dim, bags, bag, mean, sms):
     assert g.size() == known.numel()
 
 
+@pytest.mark.parametrize("general", [False, True])
+def test_keys_that_get_their_row_between_pull_and_push(general):
+    """The pull finds the row pool exhausted; the table then has room again and the keys are set. The push updates them."""
+    g, c = pair(16, "sum", 8192, slab_shift=11)
+    g.reserve(2048, exact=True)
+    mem = g.memory_usage()
+    g.table.set_limits(mem, mem)
+    keys = batch(5200, [2000, 40, 2], 13)               # 3161 distinct keys, 2048 rows
+    g.set_deterministic(general)
+    g.pull(keys.cuda()); c.pull(keys)
+    assert g.status().code() == StatusCode.OUT_OF_MEMORY
+    u = torch.unique(keys)
+    assert g.table.rows_used() == 2048 and g.size() == u.numel()
+    g.table.set_limits(0, 0)
+    g.table.set_healthy(True)
+    rows = whole(u.numel(), 16, 14)
+    g.set_rows(u.cuda(), rows.cuda(), emb_only=True); c.set_rows(u, rows, emb_only=True)
+    grads = whole(5200, 16, 15)
+    g.push(grads.cuda()); c.push(grads)
+    same_tables(g, c, keys)
+
+
 def test_lookup_of_unknown_keys_probe_chains_and_a_push_that_drops_them():
     """A nearly full index (chains of several slots), erased entries on the chains, unknown keys among the known."""
     g = SparseTable(8, "sum", device="cuda", capacity=1024, max_keys=4096, max_rows=2048, slab_shift=11, init_range=0.0)
