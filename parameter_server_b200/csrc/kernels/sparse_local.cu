@@ -94,27 +94,30 @@ __device__ __noinline__ float4 init_row4(long long key, unsigned d, unsigned lon
 
 // The grid barrier of common.cuh in two halves, so that work can stand between arriving and waiting. An error status does
 // not break it: no CTA of these kernels leaves early except on a time-out, so every call ends with its scratch clean.
-__device__ __forceinline__ unsigned grid_arrive(KernelCtl* ctl, unsigned nblocks) {
-    __syncthreads();
+// It carries one bit: whether any thread of any CTA arrived with `flag`, in the upper half of the count and then in the step
+// of the generation (a word of its own, read behind the barrier, cost every pull 0.5 to 1 us).
+__device__ __forceinline__ unsigned grid_arrive(KernelCtl* ctl, unsigned nblocks, bool flag = false) {
+    const unsigned me = __syncthreads_or(flag) ? 0x10001u : 1u;
     unsigned gen = 0;
     if (threadIdx.x == 0) {
         gen = ld_acquire_gpu(&ctl->bar_gen);
         __threadfence();
-        const unsigned arrived = atomicAdd(&ctl->bar_count, 1u) + 1u;
-        if (arrived == nblocks) {
+        const unsigned arrived = atomicAdd(&ctl->bar_count, me) + me;
+        if ((arrived & 0xffffu) == nblocks) {
             ctl->bar_count = 0;
             __threadfence();
-            atomicAdd(&ctl->bar_gen, 1u);
+            atomicAdd(&ctl->bar_gen, arrived >> 16 ? 3u : 1u);
         }
     }
     return gen;   // meaningful in thread 0
 }
-__device__ __forceinline__ bool grid_wait(KernelCtl* ctl, unsigned gen, unsigned long long limit_ns, unsigned where) {
+// `flagged` (shared memory, or null): set to that bit.
+__device__ __forceinline__ bool grid_wait(KernelCtl* ctl, unsigned gen, unsigned long long limit_ns, unsigned where, unsigned* flagged = nullptr) {
     int ok = 1;
     if (threadIdx.x == 0) {
         const unsigned long long t0 = global_timer_ns();
-        unsigned spins = 0;
-        while (ld_acquire_gpu(&ctl->bar_gen) == gen) {
+        unsigned spins = 0, now;
+        while ((now = ld_acquire_gpu(&ctl->bar_gen)) == gen) {
             if ((++spins & 63u) == 0) {
                 if (ld_acquire_gpu(&ctl->status) == kStTimeout) { ok = 0; break; }
                 if (global_timer_ns() - t0 > limit_ns) {
@@ -124,6 +127,7 @@ __device__ __forceinline__ bool grid_wait(KernelCtl* ctl, unsigned gen, unsigned
                 }
             }
         }
+        if (flagged != nullptr) *flagged = now - gen != 1u;
         __threadfence();
     }
     return __syncthreads_and(ok) != 0;
@@ -441,11 +445,10 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) local_pull_kernel(c
         }
         __syncthreads();   // the tables are emptied for the next tile
     }
-    if (reserved) cnt[7] = 1u;
     PROF_CTA(1);
-    unsigned gen = grid_arrive(a.ctl, nblocks);
-    if (!grid_wait(a.ctl, gen, a.limit_ns, W_P1)) return;
-    if (*((volatile unsigned*)&cnt[7]) != 0u) {
+    unsigned gen = grid_arrive(a.ctl, nblocks, reserved);
+    if (!grid_wait(a.ctl, gen, a.limit_ns, W_P1, &s_n)) return;
+    if (s_n != 0u) {   // a reserved key in the batch
         undo_inserts(a.table, a.new_list, a.occ, cnt + 8, a.slot_of_id, a.n);
         // reported only now: a CTA that had not started yet would take the word for an earlier call's and leave
         if (tid == 0) set_status(a.ctl, kStError, W_RESERVED_KEY);

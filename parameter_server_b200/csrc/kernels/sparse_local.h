@@ -16,8 +16,8 @@ struct LocalArgs {
     KernelCtl* ctl;
     const KernelCtl* plan_ctl;   // push: control block of the pull family
     unsigned* counters;          // [2][16] per epoch parity of the pull: 0 distinct keys, 2 occurrences listed,
-                                 // 3 work items, 5 keys with several items, 6 work items of whole CTAs, 7 a reserved key was
-                                 // met, 8 new rows and 9 new entries of the index (one 64-bit word)
+                                 // 3 work items, 5 keys with several items, 6 work items of whole CTAs, 8 new rows and
+                                 // 9 new entries of the index (one 64-bit word)
     unsigned long long limit_ns;
     unsigned long long* prof;
     unsigned long long* usage_mirror;   // pinned host words {row_bump, free_count}
